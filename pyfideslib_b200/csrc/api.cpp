@@ -187,8 +187,11 @@ fides_status fides_autotune(fides_ctx* c, int* variant, float* times_ms, int* nu
     }
     const int niv = ntt_num_inverse_variants();
     std::vector<float> fwd_ms(nv, 1e30f), inv_ms(niv, 1e30f), fwd_bms(nv, 1e30f), inv_bms(niv, 1e30f);
+    // one variant of each arithmetic (integer, double-precision) is timed; the
+    // others of that arithmetic run the same kernels
+    const int fwd_of[2] = {3, 9}, inv_of[2] = {1, 5};
     for (int r = 0; r < kRounds; ++r) {
-        for (int v = 0; v < nv; ++v) {
+        for (int v : fwd_of) {
             c->dev.ntt_variant = v;
             ntt_forward(c->dev, m, FL_PLAIN, FS_PLAIN, c->st);
             cudaEventRecord(e0, c->st);
@@ -199,7 +202,7 @@ fides_status fides_autotune(fides_ctx* c, int* variant, float* times_ms, int* nu
             for (int k = 0; k < kReps; ++k) ntt_forward(c->dev, mb, FL_PLAIN, FS_PLAIN, c->st);
             fwd_bms[v] = std::min(fwd_bms[v], elapsed() / kReps);
         }
-        for (int v = 0; v < niv; ++v) {
+        for (int v : inv_of) {
             c->dev.intt_variant = v;
             ntt_inverse(c->dev, m, IL_PLAIN, IS_PLAIN, c->st);
             cudaEventRecord(e0, c->st);
@@ -213,16 +216,15 @@ fides_status fides_autotune(fides_ctx* c, int* variant, float* times_ms, int* nu
     }
     if (tbuf) {
         // the zero residues the batched timings transformed are reused below
-        for (int v = 0; v < nv; ++v) fwd_ms[v] += fwd_bms[v];
-        for (int v = 0; v < niv; ++v) inv_ms[v] += inv_bms[v];
+        for (int v : fwd_of) fwd_ms[v] += fwd_bms[v];
+        for (int v : inv_of) inv_ms[v] += inv_bms[v];
     }
+    for (int v = 0; v < nv; ++v) fwd_ms[v] = fwd_ms[fwd_of[ntt_fwd_is_fp(v)]];
+    for (int v = 0; v < niv; ++v) inv_ms[v] = inv_ms[inv_of[ntt_inv_is_fp(v)]];
     c->tune_ms.assign(nv, 0.f);
     for (int v = 0; v < nv; ++v) c->tune_ms[v] = fwd_ms[v] + inv_ms[ntt_inverse_of(v)];
-    int best = 0, best_inv = 0;
-    for (int v = 1; v < nv; ++v)
-        if (fwd_ms[v] < fwd_ms[best]) best = v;
-    for (int v = 1; v < niv; ++v)
-        if (inv_ms[v] < inv_ms[best_inv]) best_inv = v;
+    const int best = fwd_of[fwd_ms[fwd_of[1]] < fwd_ms[fwd_of[0]]];
+    const int best_inv = inv_of[inv_ms[inv_of[1]] < inv_ms[inv_of[0]]];
     // base-conversion variants (split products need every modulus below
     // 2^60): the ModUp conversion of four top-level elements in one launch,
     // as the batched key switch runs it, in a scratch buffer freed after

@@ -32,6 +32,14 @@ __device__ __forceinline__ double fp_mulw(double y, double w, double wq, double 
     return __dadd_rn(__fma_rn(-q, p, h), l);
 }
 
+// the same plus s p, for rsub = kRint + s (s a small integer)
+__device__ __forceinline__ double fp_mulw_sh(double y, double w, double wq, double p, double rsub) {
+    const double h = __dmul_rn(y, w);
+    const double l = __fma_rn(y, w, -h);
+    const double q = __dsub_rn(__fma_rn(y, wq, kRint), rsub);
+    return __dadd_rn(__fma_rn(-q, p, h), l);
+}
+
 // x - rint(x / p) p, magnitude <= p/2 + |x| 2^-52 (|x| < 2^51)
 __device__ __forceinline__ double fp_center(double x, double p, double pinv) {
     const double q = __dsub_rn(__fma_rn(x, pinv, kRint), kRint);
@@ -48,6 +56,23 @@ __device__ __forceinline__ uint64_t fp_to_u(double v, double p, double pinv_up) 
     const double b = __dadd_rn(v, __dadd_rn(two_p, kTwo52));  // a + 2^52, exact
     const double q = __dsub_rn(__fma_rd(a, pinv_up, kRint), kRint);
     return as_u64(__fma_rn(-q, p, b)) & kMant52;  // (a - q p) + 2^52 -> low 52 bits
+}
+
+// the same for v in (0, 4p)
+__device__ __forceinline__ uint64_t fp_pos_to_u(double v, double p, double pinv_up) {
+    const double q = __dsub_rn(__fma_rd(v, pinv_up, kRint), kRint);
+    return as_u64(__dadd_rn(__fma_rn(-q, p, v), kTwo52)) & kMant52;
+}
+
+// the same for |v| < 8p: centred around p first
+__device__ __forceinline__ uint64_t fp_sum_to_u(double v, double p, double pinv_up) {
+    const double q = __dsub_rn(__fma_rn(v, pinv_up, kRint), kRint + 1.0);
+    return fp_pos_to_u(__fma_rn(-q, p, v), p, pinv_up);
+}
+
+// a constant residue c < p as a double in (-p/2, p/2]
+__device__ __forceinline__ double fp_centred_const(uint64_t c, uint64_t p) {
+    return c > (p >> 1) ? -(double)(p - c) : (double)c;
 }
 
 // x y mod p up to a multiple of p for residues x, y < p < 2^50 (pinv >= 1/p,

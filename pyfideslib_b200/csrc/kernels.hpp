@@ -24,6 +24,21 @@ enum { IS_PLAIN = 0, IS_MODUP = 1, IS_MODDOWN = 2 };
 uint64_t launch_count();
 void count_launches(int n);
 
+// the transforms of one ring dimension (ntt_n.cu)
+struct KsFuseArgs;
+struct NttOps {
+    void (*fwd)(const DevCtx&, const LimbMap&, cudaStream_t);
+    void (*inv)(const DevCtx&, const LimbMap&, cudaStream_t);
+    void (*fwd_cols)(const DevCtx&, const LimbMap&, cudaStream_t);
+    void (*rows_ks)(const DevCtx&, const KsFuseArgs&, int nb, cudaStream_t);
+    void (*prepare)(const DevCtx&);
+};
+template <int LOGN>
+const NttOps& ntt_ops();
+// arithmetic of a forward variant / an inverse configuration (see ntt.cu)
+bool ntt_fwd_is_fp(int variant);
+bool ntt_inv_is_fp(int variant);
+
 bool ntt_supported(int logN);
 int ntt_num_variants();
 int ntt_num_inverse_variants();
