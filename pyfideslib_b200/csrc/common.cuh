@@ -62,8 +62,8 @@ struct DevCtx {
     const PrimeConst* pc;        // [L+K]
     const uint64_t* fwd_tw;      // [L+K][N][2]  psi^{bitrev(i)}, companion
     const uint64_t* inv_tw;      // [L+K][N][2]  psi^{-bitrev(i)}, companion
-    const uint64_t* fwd_twf;     // [L+K][N][2]  bit patterns of the doubles w = psi^{bitrev(i)} and w / p
-                                 //              (primes below 2^50; zero rows otherwise)
+    const uint64_t* fwd_twf;     // [L+K][N][2]  bit patterns of the doubles w = psi^{bitrev(i)}, centred in
+                                 //              (-p/2, p/2], and w / p (primes below 2^50; zero rows otherwise)
     const uint64_t* inv_twf;     // [L+K][N][2]  the same for psi^{-bitrev(i)}
     const uint64_t* intt_scale;  // [L+K][4]     s=N^-1, s', s*w1, (s*w1)'  (w1 = inverse twiddle 1)
     const uint64_t* modup_scale; // [L][L][4]    same with s = N^-1 * (Q'/q_i)^-1 for level, prime

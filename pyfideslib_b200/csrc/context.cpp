@@ -352,14 +352,17 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
             I[2 * j] = b[r];
             I[2 * j + 1] = shoup_precompute(b[r], pr);
         }
-        // double-precision butterflies (primes below 2^50): w and the
-        // correctly rounded quotient w / p
+        // double-precision butterflies (primes below 2^50): w centred in
+        // (-p/2, p/2] (its products then take operands up to 4p, see
+        // ntt_sched.hpp) and the correctly rounded quotient w / p
         if (pr < kFpPrimeBound) {
             k.pinv_f64 = f64_bits(recip_up(pr));
             uint64_t* D = fwdf.data() + (size_t)i * N * 2;
             uint64_t* E = invf.data() + (size_t)i * N * 2;
             for (int j = 0; j < N; ++j) {
-                const double w = (double)F[2 * j], v = (double)I[2 * j];
+                const uint64_t half = pr >> 1;
+                const double w = F[2 * j] > half ? -(double)(pr - F[2 * j]) : (double)F[2 * j];
+                const double v = I[2 * j] > half ? -(double)(pr - I[2 * j]) : (double)I[2 * j];
                 D[2 * j] = f64_bits(w);
                 D[2 * j + 1] = f64_bits(w / (double)pr);
                 E[2 * j] = f64_bits(v);

@@ -495,8 +495,8 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
 //
 // Sums: for primes below 2^50 with fp_sums, each product is an exact FP64
 // fp_mulmod of a transformed value (below 1.7p: the last row stage centres) or
-// the own limb (< p) with a key residue (< p): |r| <= 1.14p, and up to 6 digits
-// sum below 6.9p < 2^53; otherwise products are accumulated in 128 bits.
+// the own limb (< p) with a key residue (< p): |r| <= (1/2 + 1.7 * 3/8) p, and
+// up to 6 digits sum below 6.9p < 2^53; otherwise products are accumulated in 128 bits.
 // Results are canonical residues, identical to k_ks_inner's.
 //
 // MB: CTAs of four warps per SM the register budget is cut for (6, or 4 where
