@@ -286,10 +286,31 @@ __global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
     uint64_t x[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) x[k] = lr.in[(size_t)(th + (k << (LR - 4))) * C + col];
+    const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
     if (lr.lmode == FL_SWITCHMOD) {
         const uint64_t om = ctx.pc[lr.level].p;
+        if (fp && om < kFpPrimeBound) {
+            // the centred lift of a residue mod om is already an operand the
+            // butterflies take while om <= 2p
+            const double omd = __ull2double_rn(om);
+            const bool wide = om > pc.two_p;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) x[k] = switch_modulus(x[k], om, pc);
+            for (int k = 0; k < 16; ++k) {
+                double v = as_f64(fp_from_u(x[k]));
+                if (x[k] > (om >> 1)) v = __dsub_rn(v, omd);
+                if (wide) v = fp_center(v, p, pinv);
+                x[k] = as_u64(v);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                x[k] = switch_modulus(x[k], om, pc);
+                if (fp) x[k] = fp_from_u(x[k]);
+            }
+        }
+    } else if (fp) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) x[k] = fp_from_u(x[k]);
     }
     stage_wait();
     __syncthreads();
@@ -297,11 +318,8 @@ __global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
     auto g1 = [&](int kb, int g) { return tws[(8 >> kb) + g]; };
     // stages 4..LR-1: r = 16 th + k
     auto g2 = [&](int kb, int g) { return tws[(1 << (LR - 1 - kb)) + (th << (3 - kb)) + g]; };
-    const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
     const bool approx = pc.p < kApproxPrimeBound;
     if (fp) {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) x[k] = fp_from_u(x[k]);
         fp_fwd<LOGN, LR, 0, 3>(x, g1, p, pinv, kRint);
     } else {
         int_fwd<3>(approx, x, g1, pc.p, pc.two_p);
@@ -388,28 +406,21 @@ struct RowFwd {
     }
 };
 
-// v: canonical NTT value of word g (limb offset)
-__device__ __forceinline__ uint64_t fwd_epilogue(const DevCtx& ctx, const LimbRef& lr, const PrimeConst& pc, size_t g,
-                                                 uint64_t v) {
-    switch (lr.smode) {
-        case FS_MODDOWN: {
-            const ulonglong2 pinv = ldg2(ctx.md_pinv, lr.prime);
-            uint64_t r = mul_shoup(sub_mod(lr.in2[g], v, pc.p), pinv.x, pinv.y, pc.p);
-            if (lr.in3) r = add_mod(r, lr.in3[g], pc.p);
-            return r;
-        }
-        case FS_RESCALE: {
-            const ulonglong2 qi = ldg2(ctx.rs_qinv, (size_t)lr.level * ctx.L + lr.prime);
-            return mul_shoup(sub_mod(lr.in2[g], v, pc.p), qi.x, qi.y, pc.p);
-        }
-        case FS_MDRS: {
-            const ulonglong2 pinv = ldg2(ctx.md_pinv, lr.prime);
-            const ulonglong2 qi = ldg2(ctx.rs_qinv, (size_t)lr.level * ctx.L + lr.prime);
-            const uint64_t u = add_mod(lr.in3[g], mul_shoup(lr.in2[g], pinv.x, pinv.y, pc.p), pc.p);
-            return mul_shoup(sub_mod(u, v, pc.p), qi.x, qi.y, pc.p);
-        }
-        default:
-            return v;
+// The epilogue of one warp's tile: out[i] = f(value, in2[i], in3[i]) over the
+// words of the tile, two adjacent words per lane and step (16-byte accesses).
+// NIN: operands read (in3 may be null: reads as 0).
+template <class G, int NIN, class F>
+__device__ __forceinline__ void row_epilogue(const LimbRef& lr, size_t base, const uint64_t* sw, int lane, F f) {
+#pragma unroll 4
+    for (int j = 0; j < 8; ++j) {
+        const int i = 2 * lane + 2 * G::WL * j;
+        const int wi = padi(i);
+        ulonglong2 a = make_ulonglong2(0, 0), b = a, o;
+        if (NIN > 0) a = *reinterpret_cast<const ulonglong2*>(lr.in2 + base + i);
+        if (NIN > 1 && lr.in3) b = *reinterpret_cast<const ulonglong2*>(lr.in3 + base + i);
+        o.x = f(sw[wi], a.x, b.x);
+        o.y = f(sw[wi + 1], a.y, b.y);
+        *reinterpret_cast<ulonglong2*>(lr.out + base + i) = o;
     }
 }
 
@@ -450,31 +461,67 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
     stage_wait();
     __syncwarp(G::MASK);
     const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
+    // double-precision limbs end within 1.63p of 0, or of 2p when the value
+    // is reduced as it is
     if (fp)
-        rf.run_fp(x, sw, s_tw, lane, th, rl, p, pinv, kRint + 2.0);  // ends in (0, 4p)
+        rf.run_fp(x, sw, s_tw, lane, th, rl, p, pinv, lr.smode == FS_PLAIN ? kRint + 2.0 : kRint);
     else
         rf.run_int(x, sw, s_tw, twg, row0 + rl, lane, th, rl, pc);
     __syncwarp(G::MASK);
 #pragma unroll
     for (int k = 0; k < 16; ++k) sw[17 * lane + k] = x[k];
     __syncwarp(G::MASK);
-#pragma unroll 4
-    for (int j = 0; j < 8; ++j) {
-        const int i = 2 * lane + 2 * G::WL * j;
-        const int wi = padi(i);
-        uint64_t v0 = sw[wi], v1 = sw[wi + 1];
-        if (fp) {
-            v0 = fp_pos_to_u(as_f64(v0), p, pinv);
-            v1 = fp_pos_to_u(as_f64(v1), p, pinv);
-        } else {
-            v0 = reduce_fwd(v0, pc);
-            v1 = reduce_fwd(v1, pc);
-        }
-        ulonglong2 o;
-        o.x = fwd_epilogue(ctx, lr, pc, base + i, v0);
-        o.y = fwd_epilogue(ctx, lr, pc, base + i + 1, v1);
-        *reinterpret_cast<ulonglong2*>(lr.out + base + i) = o;
+    if (fp) {
+        // the combinations stay on the FP64 pipes: operands are residues (or
+        // sums below 3.2p), the constants are centred with exact companions, so
+        // every product is below 0.62p and the last one, shifted by p, is
+        // positive.  (64-bit Shoup products here cost as many issue slots as the
+        // butterflies: the final row pass of 32 products took 925 us, 58 x 32 limbs.)
+        const double2 ci = lr.smode == FS_PLAIN || lr.smode == FS_RESCALE
+                               ? make_double2(0, 0)
+                               : *reinterpret_cast<const double2*>(ctx.md_pinvf + 2 * lr.prime);
+        const double2 cq = lr.smode == FS_RESCALE || lr.smode == FS_MDRS
+                               ? *reinterpret_cast<const double2*>(ctx.rs_qinvf + 2 * ((size_t)lr.level * ctx.L + lr.prime))
+                               : make_double2(0, 0);
+        auto conv = [](uint64_t u) { return as_f64(fp_from_u(u)); };
+        if (lr.smode == FS_PLAIN)
+            row_epilogue<G, 0>(lr, base, sw, lane,
+                               [&](uint64_t v, uint64_t, uint64_t) { return fp_pos_to_u(as_f64(v), p, pinv); });
+        else if (lr.smode == FS_MODDOWN)
+            row_epilogue<G, 2>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t b) {
+                const double t = fp_mulw_sh(__dsub_rn(conv(a), as_f64(v)), ci.x, ci.y, p, kRint + 1.0);
+                return fp_pos_to_u(__dadd_rn(t, conv(b)), p, pinv);
+            });
+        else if (lr.smode == FS_RESCALE)
+            row_epilogue<G, 1>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t) {
+                return fp_pos_to_u(fp_mulw_sh(__dsub_rn(conv(a), as_f64(v)), cq.x, cq.y, p, kRint + 1.0), p, pinv);
+            });
+        else
+            row_epilogue<G, 2>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t b) {
+                const double u = __dadd_rn(conv(b), fp_mulw(conv(a), ci.x, ci.y, p));
+                return fp_pos_to_u(fp_mulw_sh(__dsub_rn(u, as_f64(v)), cq.x, cq.y, p, kRint + 1.0), p, pinv);
+            });
+        return;
     }
+    const ulonglong2 ci = lr.smode == FS_PLAIN || lr.smode == FS_RESCALE ? make_ulonglong2(0, 0) : ldg2(ctx.md_pinv, lr.prime);
+    const ulonglong2 cq = lr.smode == FS_RESCALE || lr.smode == FS_MDRS
+                              ? ldg2(ctx.rs_qinv, (size_t)lr.level * ctx.L + lr.prime)
+                              : make_ulonglong2(0, 0);
+    if (lr.smode == FS_PLAIN)
+        row_epilogue<G, 0>(lr, base, sw, lane, [&](uint64_t v, uint64_t, uint64_t) { return reduce_fwd(v, pc); });
+    else if (lr.smode == FS_MODDOWN)
+        row_epilogue<G, 2>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t b) {
+            return add_mod(mul_shoup(sub_mod(a, reduce_fwd(v, pc), pc.p), ci.x, ci.y, pc.p), b, pc.p);
+        });
+    else if (lr.smode == FS_RESCALE)
+        row_epilogue<G, 1>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t) {
+            return mul_shoup(sub_mod(a, reduce_fwd(v, pc), pc.p), cq.x, cq.y, pc.p);
+        });
+    else
+        row_epilogue<G, 2>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t b) {
+            const uint64_t u = add_mod(b, mul_shoup(a, ci.x, ci.y, pc.p), pc.p);
+            return mul_shoup(sub_mod(u, reduce_fwd(v, pc), pc.p), cq.x, cq.y, pc.p);
+        });
 }
 
 // ---------------------------------------------------------------------------
@@ -677,6 +724,7 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
         for (int kb = 0; kb < NST2; ++kb)
             D[kb] = ldg2(twg, ((size_t)(G::R + row) << (LC - 1 - kb)) + ((size_t)th << (3 - kb)));
     }
+    const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
     uint64_t x[16];
     {
         // all 16 words of the lane are loaded before any is used, so the
@@ -685,36 +733,45 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
         const uint64_t* in = lr.in + base + 2 * lane;
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = *reinterpret_cast<const ulonglong2*>(in + 2 * G::WL * q);
-        if (lr.lmode != IL_PLAIN) {
+        if (lr.lmode == IL_PLAIN) {
+            if (fp) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    v[q].x = fp_from_u(v[q].x);
+                    v[q].y = fp_from_u(v[q].y);
+                }
+            }
+        } else {
             const uint64_t* in2 = lr.in2 + base + 2 * lane;
-            if (lr.lmode == IL_MUL) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(in2 + 2 * G::WL * q);
-                    v[q].x = mul_mod(v[q].x, u.x, pc);
-                    v[q].y = mul_mod(v[q].y, u.y, pc);
+            const bool mul = lr.lmode == IL_MUL;
+            // double-precision limbs: exact products, centred (the schedule's entry bound)
+            const double2 cf = fp && !mul ? *reinterpret_cast<const double2*>(ctx.md_pinvf + 2 * lr.prime) : make_double2(0, 0);
+            const ulonglong2 pi = !fp && !mul ? ldg2(ctx.md_pinv, lr.prime) : make_ulonglong2(0, 0);
+            auto one = [&](uint64_t a, uint64_t b) -> uint64_t {
+                if (fp) {
+                    const double x = as_f64(fp_from_u(a)), y = as_f64(fp_from_u(b));
+                    const double r = mul ? fp_mulmod(x, y, p, pinv) : __dadd_rn(x, fp_mulw(y, cf.x, cf.y, p));
+                    return as_u64(fp_center(r, p, pinv));
                 }
-            } else {
-                const ulonglong2 pi = ldg2(ctx.md_pinv, lr.prime);
+                return mul ? mul_mod(a, b, pc) : add_mod(a, mul_shoup(b, pi.x, pi.y, pc.p), pc.p);
+            };
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(in2 + 2 * G::WL * q);
-                    v[q].x = add_mod(v[q].x, mul_shoup(u.x, pi.x, pi.y, pc.p), pc.p);
-                    v[q].y = add_mod(v[q].y, mul_shoup(u.y, pi.x, pi.y, pc.p), pc.p);
-                }
+            for (int q = 0; q < 8; ++q) {
+                const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(in2 + 2 * G::WL * q);
+                v[q].x = one(v[q].x, u.x);
+                v[q].y = one(v[q].y, u.y);
             }
         }
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int wi = padi(2 * lane + 2 * G::WL * q);
-            sw[wi] = fp ? fp_from_u(v[q].x) : v[q].x;
-            sw[wi + 1] = fp ? fp_from_u(v[q].y) : v[q].y;
+            sw[wi] = v[q].x;
+            sw[wi + 1] = v[q].y;
         }
     }
     stage_wait();
     __syncwarp(G::MASK);
 
-    const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
     if constexpr (NST2 > 0) {
 #pragma unroll
         for (int k = 0; k < 16; ++k) x[k] = sw[17 * lane + k];
