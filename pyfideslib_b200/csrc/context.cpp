@@ -355,8 +355,8 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
         // double-precision butterflies (primes below 2^50): w centred in
         // (-p/2, p/2] (its products then take operands up to 4p, see
         // ntt_sched.hpp) and the correctly rounded quotient w / p
+        k.pinv_f64 = f64_bits(pr < kFpPrimeBound ? recip_up(pr) : 1.0 / (double)pr);
         if (pr < kFpPrimeBound) {
-            k.pinv_f64 = f64_bits(recip_up(pr));
             uint64_t* D = fwdf.data() + (size_t)i * N * 2;
             uint64_t* E = invf.data() + (size_t)i * N * 2;
             for (int j = 0; j < N; ++j) {

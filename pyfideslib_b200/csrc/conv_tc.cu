@@ -20,10 +20,10 @@
 // A tile of 128 coefficients is multiplied by B with tcgen05.mma kind::i8
 // (M = 128, N = 8 columns per target, K = 32 bytes per instruction) into
 // tensor memory; the epilogue reads each coefficient's column sums with
-// tcgen05.ld, reassembles V' and reduces it with one Barrett step
-// (q = floor(floor(V'/2^16) floor(2^80/p) / 2^64), remainder in [0, 2p)).
-// The tensor cores take the 64x64-bit products off the integer pipes; what
-// is left there is a few shifts and adds and one 64-bit quotient per output.
+// tcgen05.ld, reassembles V' and reduces it with one 15-bit quotient
+// (reduce_cols).  The tensor cores take the 64x64-bit products off the integer
+// pipes; what is left there is a few shifts and adds and three multiplies per
+// output.
 //
 // Operands sit in shared memory in the canonical K-major layout without
 // swizzle: core matrices of 8 rows x 16 bytes stored contiguously, 8-row
@@ -89,13 +89,20 @@ __device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t phase) {
     return false;
 }
 
-// 16 consecutive accumulator columns of this thread's lane (no wait)
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&c)[16]) {
+// 8 and 32 consecutive accumulator columns of this thread's lane (no wait)
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&c)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&c)[32]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-        "%14, %15}, [%16];\n"
-        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7]),
-          "=r"(c[8]), "=r"(c[9]), "=r"(c[10]), "=r"(c[11]), "=r"(c[12]), "=r"(c[13]), "=r"(c[14]), "=r"(c[15])
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7]), "=r"(c[8]),
+          "=r"(c[9]), "=r"(c[10]), "=r"(c[11]), "=r"(c[12]), "=r"(c[13]), "=r"(c[14]), "=r"(c[15]), "=r"(c[16]),
+          "=r"(c[17]), "=r"(c[18]), "=r"(c[19]), "=r"(c[20]), "=r"(c[21]), "=r"(c[22]), "=r"(c[23]), "=r"(c[24]),
+          "=r"(c[25]), "=r"(c[26]), "=r"(c[27]), "=r"(c[28]), "=r"(c[29]), "=r"(c[30]), "=r"(c[31])
         : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
@@ -104,17 +111,39 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 // The pairs w_k = c_{2k} + c_{2k+1} 2^8 fit 32 bits, and with
 // e = w_0 + w_2 2^32, o = w_1 + w_3 2^32:  V' = e + o 2^16,
 // floor(V'/2^16) = floor(e/2^16) + o  and  V' mod 2^64 = e + (o << 16).
-// V' < 2^79.01, so with mu = floor(2^80/p) the Barrett quotient
-// q = floor(floor(V'/2^16) mu / 2^64) is floor(V'/p) or one less, and
-// V' - q p (formed modulo 2^64) lies in [0, 2p).
-__device__ __forceinline__ uint64_t reduce_cols(const uint32_t* c, uint64_t mu, uint64_t p) {
+// V' < 8 cnt 255 p (cnt input limbs): the quotient has at most 15 bits, so 32
+// bits T = floor(V' / 2^s) of V' and one 32-bit high product give it,
+//   q = floor(T M / 2^(32+k)),  M = floor(2^(32+k+s) / p) or one less,
+// with s = max(16, bits(p) + bits(2040 cnt) - 32), k = bits(p) - 1 - s: short of
+// V'/p by less than 1 + 2^s / p + 2 T / 2^(32+k) < 2, so V' - q p (formed modulo
+// 2^64) lies in [0, 2p).  (A 64-bit Barrett quotient, floor(2^80 / p), took
+// eight half-rate multiplies per output against three, and that pipe was 65%
+// busy: ModUp of 32 elements 608 us, ModDown 598 us at the HMult shape.)
+struct __align__(16) TcMod {
+    uint64_t np;   // -p
+    uint32_t M;
+    uint32_t shk;  // s - 16, and k << 16
+};
+__device__ __forceinline__ TcMod tc_mod(const PrimeConst& pc, int cnt) {
+    const int bits = 64 - __clzll((long long)pc.p);
+    const int s = max(16, bits + (32 - __clz(2040 * cnt)) - 32);
+    const int k = max(0, bits - 1 - s);
+    // 1/p is within 2^-52 relative: one less than its floor never exceeds the exact floor
+    const double m = ldexp(__longlong_as_double((long long)pc.pinv_f64), 32 + k + s);
+    return {0 - pc.p, (uint32_t)(uint64_t)m - 1u, (uint32_t)(s - 16) | (uint32_t)k << 16};
+}
+__device__ __forceinline__ uint64_t reduce_cols(const uint32_t* c, const TcMod& t) {
     const uint32_t w0 = c[0] + (c[1] << 8), w1 = c[2] + (c[3] << 8);
     const uint32_t w2 = c[4] + (c[5] << 8), w3 = c[6] + (c[7] << 8);
     const uint64_t e = ((uint64_t)w2 << 32) | w0;
     const uint64_t o = ((uint64_t)w3 << 32) | w1;
-    const uint64_t q = __umul64hi((e >> 16) + o, mu);
-    const uint64_t r = e + (o << 16) - q * p;
-    return r >= p ? r - p : r;
+    const uint64_t h = (e >> 16) + o;
+    const uint32_t T = __funnelshift_r((uint32_t)h, (uint32_t)(h >> 32), t.shk);  // shift taken mod 32
+    const uint32_t q = __umulhi(T, t.M) >> (t.shk >> 16);
+    const uint64_t a = (uint64_t)q * (uint32_t)t.np + e;
+    const uint64_t r = a + ((uint64_t)(q * (uint32_t)(t.np >> 32)) << 32) + (o << 16);
+    const uint64_t s = r + t.np;
+    return (int64_t)s < 0 ? r : s;  // r < 2p < 2^63
 }
 
 // target index m of a digit -> prime id (the other Q primes, then the special ones)
@@ -262,17 +291,17 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
     uint8_t* sA = smem;                                   // 2*CK chunks x kTcLboA
     uint8_t* sB = smem + 2 * CK * kTcLboA;                // 2*CK chunks x lbo_b
     PrimeConst* sP = reinterpret_cast<PrimeConst*>(sB + 2 * CK * lbo_b);
-    uint64_t* sMu = reinterpret_cast<uint64_t*>(sP + ntar2);       // floor(2^80 / p) per target
-    uint64_t* sOm = sMu + ntar2;                         // ModDown: q_level mod target
+    TcMod* sMod = reinterpret_cast<TcMod*>(sP + ntar2);  // reduction constants per target
+    uint64_t* sOm = reinterpret_cast<uint64_t*>(sMod + ntar2);  // ModDown: target - q_level mod target
     uint64_t* sTL = sOm + (MD ? ntar2 : 0);               // ModDown: tl per row
     uint64_t* bar = sTL + (MD ? kTcRows : 0);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
 
-    for (int m = threadIdx.x; m < ntar; m += kTcThreads) {
-        const PrimeConst pc = ctx.pc[sh.tprime(ctx, m)];
+    for (int m = threadIdx.x; m < ntar2; m += kTcThreads) {  // (the pad target: any constants)
+        const PrimeConst pc = ctx.pc[sh.tprime(ctx, min(m, ntar - 1))];
         sP[m] = pc;
-        sMu[m] = (uint64_t)(((unsigned __int128)1 << 80) / pc.p);
-        if (MD) sOm[m] = csub(reduce64_lazy(ctx.pc[level].p, pc), pc.p);
+        sMod[m] = tc_mod(pc, cnt);
+        if (MD) sOm[m] = pc.p - csub(reduce64_lazy(ctx.pc[level].p, pc), pc.p);
     }
     // A: zero once (limbs cnt..4*CK-1 stay zero)
     for (int i = threadIdx.x; i < 2 * CK * (int)kTcLboA / 16; i += kTcThreads)
@@ -321,29 +350,26 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
             if (e < cnt * kTcRows) pre[q] = src[(size_t)(e / kTcRows) * ctx.N + e % kTcRows];
         }
     };
-    auto value = [&](const uint32_t* c, int m) { return reduce_cols(c, sMu[m], sP[m].p); };
     if (it_begin < it_end) fetch(it_begin);
     for (int it = it_begin; it < it_end && ok; ++it) {
         int half;
         const size_t boff = item_off(it, half);
         const size_t j = (size_t)(it % ntiles) * kTcRows + row;  // this thread's coefficient
-        // output of target m for this thread's row (v = conversion value mod p_m)
+        // this row's outputs: target m at obase + m N (the fused ModDown's target 0
+        // is the top limb, which has none)
+        uint64_t* obase = MD ? args.md.w[half] + boff + j - (fused ? ctx.N : 0)
+                             : args.dig + boff + (size_t)d * args.dig_stride * ctx.N + j;
+        uint64_t tl = 0, ql = 0;
+        bool up = false;  // tl stands for tl - q_l
         auto finish = [&](int m, uint64_t v) {
-            if (MD) {
-                if (fused) {
-                    // v = P^-1 conv_q (folded into the constants)
-                    // SwitchModulus(tl, q_l -> q) with q_l mod q precomputed
-                    const PrimeConst pc = sP[m];
-                    const uint64_t tl = sTL[row], ql = sP[0].p;
-                    uint64_t sw = tl > (ql >> 1) ? tl + (pc.p - sOm[m]) : tl;
-                    if (pc.p < ql) sw = csub(reduce64_lazy(sw, pc), pc.p);
-                    args.md.w[half][boff + (size_t)(m - 1) * ctx.N + j] = add_mod(v, sw, pc.p);
-                } else {
-                    args.md.w[half][boff + (size_t)m * ctx.N + j] = v;
-                }
-            } else {
-                args.dig[boff + ((size_t)d * args.dig_stride + m) * ctx.N + j] = v;
+            if (MD && fused) {
+                // v = P^-1 conv_q (folded into the constants); SwitchModulus(tl, q_l -> q)
+                const PrimeConst pc = sP[m];
+                uint64_t sw = up ? tl + sOm[m] : tl;
+                if (pc.p < ql) sw = csub(reduce64_lazy(sw, pc), pc.p);
+                v = add_mod(v, sw, pc.p);
             }
+            obase[(size_t)((uint32_t)m * (uint32_t)ctx.N)] = v;
         };
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
@@ -380,40 +406,42 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             // the next item's limbs load while this chunk's outputs are formed
             if (m0 + CHUNK >= ntar2 && it + 1 < it_end) fetch(it + 1);
-            // target pairs (2p, 2p+1) share one 16-column load; warps of half
-            // wh take pairs wh, wh+2, ... two at a time
-            int first = wh;
-            if (MD && fused && m0 == 0) {
-                // pair 0 holds the top limb: every row's tl first, shared through smem
-                uint32_t c[16];
-                uint64_t v1 = 0;
-                if (wh == 0) {
-                    tmem_ld16(t_lane, c);
-                    tmem_wait_ld();
-                    const uint64_t ql = sP[0].p;
-                    sTL[row] = sub_mod(args.md.ttop[half][boff + j], value(c, 0), ql);  // ttop - P^-1 conv_l
-                    if (ntar > 1) v1 = value(c + 8, 1);
+            if (MD && fused) {
+                if (m0 == 0) {
+                    // target 0 is the top limb: every row's tl first, shared through smem
+                    if (wh == 0) {
+                        uint32_t c[8];
+                        tmem_ld8(t_lane, c);
+                        tmem_wait_ld();
+                        sTL[row] = sub_mod(args.md.ttop[half][boff + j], reduce_cols(c, sMod[0]), sP[0].p);
+                    }
+                    __syncthreads();
                 }
-                __syncthreads();
-                if (wh == 0) {
-                    if (ntar > 1) finish(1, v1);
-                    first = 2;
-                }
+                tl = sTL[row];
+                ql = sP[0].p;
+                up = tl > (ql >> 1);
             }
-            for (int pp = first; 2 * pp < nt; pp += 4) {
-                const bool two = 2 * (pp + 2) < nt;
-                uint32_t c0[16], c1[16];
-                tmem_ld16(t_lane + (uint32_t)(2 * pp * kTcCols), c0);
-                if (two) tmem_ld16(t_lane + (uint32_t)(2 * (pp + 2) * kTcCols), c1);
+            // four targets share one 32-column load (columns past nt hold old
+            // sums, their values are dropped); the warps of half wh take every
+            // second group.  The four reductions are independent and run before
+            // any store, so that their latencies overlap: with branches between
+            // them the epilogue waited two issue slots per instruction at 16
+            // warps per SM.
+#pragma unroll 1
+            for (int g = 4 * wh; g < nt; g += 8) {
+                uint32_t c[32];
+                tmem_ld32(t_lane + (uint32_t)(g * kTcCols), c);
+                const int m = m0 + g;
+                TcMod md[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) md[u] = sMod[min(m + u, ntar2 - 1)];
                 tmem_wait_ld();
-                const int m = m0 + 2 * pp;
-                finish(m, value(c0, m));
-                if (m + 1 < ntar) finish(m + 1, value(c0 + 8, m + 1));
-                if (two) {
-                    const int m2 = m + 4;
-                    finish(m2, value(c1, m2));
-                    if (m2 + 1 < ntar) finish(m2 + 1, value(c1 + 8, m2 + 1));
-                }
+                uint64_t v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = reduce_cols(c + 8 * u, md[u]);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (g + u < nt && m + u < ntar && !(MD && fused && m + u == 0)) finish(m + u, v[u]);
             }
         }
     }
@@ -431,7 +459,7 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
 // dynamic shared memory of one CTA for ntar targets
 size_t tc_smem_bytes(int ck, int ntar, bool md) {
     const size_t t2 = (size_t)((ntar + 1) & ~1);
-    return (size_t)2 * ck * kTcLboA + (size_t)2 * ck * t2 * kTcCols / 8 * 128 + t2 * (sizeof(PrimeConst) + 8) +
+    return (size_t)2 * ck * kTcLboA + (size_t)2 * ck * t2 * kTcCols / 8 * 128 + t2 * (sizeof(PrimeConst) + sizeof(TcMod)) +
            (md ? t2 * 8 + (size_t)kTcRows * 8 : 0) + 16;
 }
 

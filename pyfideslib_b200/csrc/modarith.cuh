@@ -42,7 +42,7 @@ struct PrimeConst {
     uint64_t r64_sh;  // Shoup companion of r64
     uint64_t ninv;    // N^-1 mod p
     uint64_t ninv_sh;
-    uint64_t pinv_f64;  // bit pattern of the double 1/p rounded up (p < 2^50; 0 otherwise)
+    uint64_t pinv_f64;  // bit pattern of the double 1/p (rounded up for p < 2^50)
 };
 
 // Forward transforms of primes below this bound run their butterflies on the
