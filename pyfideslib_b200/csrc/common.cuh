@@ -80,6 +80,17 @@ struct DevCtx {
     uint32_t* err;               // the context's device error word (kDevErr* bits)
 };
 
+#if defined(__CUDACC__)
+// Programmatic dependent launch: the library's kernels are launched so that
+// their CTAs may start while the previous kernel of the stream drains
+// (launch_pdl, kernels.hpp).  A kernel reads or writes nothing that an earlier
+// kernel produces or uses before pdl_wait (only context tables and switching
+// keys' addresses), and every CTA passes pdl_wait, so completion stays
+// transitive along the stream.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+#endif
+
 // A launch covers up to kMaxSeg segments of contiguous limbs.  Within a
 // segment, limb i (0 <= i < count) sits at in/out + i*N and maps to prime
 //   j = i < skip_lo ? i : i + skip_cnt;   prime = j < nq ? q0 + j : L + (j - nq).

@@ -260,6 +260,7 @@ template <int CK, int CHUNK, bool MD>
 __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
     k_conv_tc(const __grid_constant__ DevCtx ctx, int level, const __grid_constant__ TcArgs args) {
     extern __shared__ __align__(1024) uint8_t smem[];
+    pdl_trigger();
     const int ntiles = ctx.N / kTcRows;
     // ModDown with the top limb (target 0 = prime `level`); both halves alike
     const bool fused = MD && args.md.ttop[0] != nullptr;
@@ -350,6 +351,9 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
             if (e < cnt * kTcRows) pre[q] = src[(size_t)(e / kTcRows) * ctx.N + e % kTcRows];
         }
     };
+    // everything up to here (tables, tensor memory, barrier) may run under the
+    // previous kernel's tail
+    pdl_wait();
     if (it_begin < it_end) fetch(it_begin);
     for (int it = it_begin; it < it_end && ok; ++it) {
         int half;
@@ -479,19 +483,19 @@ void launch_ck(int ck, dim3 g, size_t smem, const DevCtx& ctx, int level, const 
     switch (ck) {
         case 1:
             set_smem_attr<1, CHUNK, MD>();
-            k_conv_tc<1, CHUNK, MD><<<g, kTcThreads, smem, st>>>(ctx, level, a);
+            launch_pdl(k_conv_tc<1, CHUNK, MD>, g, kTcThreads, smem, st, ctx, level, a);
             break;
         case 2:
             set_smem_attr<2, CHUNK, MD>();
-            k_conv_tc<2, CHUNK, MD><<<g, kTcThreads, smem, st>>>(ctx, level, a);
+            launch_pdl(k_conv_tc<2, CHUNK, MD>, g, kTcThreads, smem, st, ctx, level, a);
             break;
         case 3:
             set_smem_attr<3, CHUNK, MD>();
-            k_conv_tc<3, CHUNK, MD><<<g, kTcThreads, smem, st>>>(ctx, level, a);
+            launch_pdl(k_conv_tc<3, CHUNK, MD>, g, kTcThreads, smem, st, ctx, level, a);
             break;
         default:
             set_smem_attr<4, CHUNK, MD>();
-            k_conv_tc<4, CHUNK, MD><<<g, kTcThreads, smem, st>>>(ctx, level, a);
+            launch_pdl(k_conv_tc<4, CHUNK, MD>, g, kTcThreads, smem, st, ctx, level, a);
             break;
     }
 }

@@ -1,5 +1,6 @@
 // kernels.hpp -- host-side launchers of the sm_100a kernels.
 #pragma once
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -19,6 +20,31 @@ enum {
 enum { IL_PLAIN = 0, IL_MUL = 1, IL_AXPY_PINV = 2 };
 // inverse-NTT epilogues (pass B scale): N^-1 times 1 / ModUp hat-inverse / ModDown hat-inverse
 enum { IS_PLAIN = 0, IS_MODUP = 1, IS_MODDOWN = 2 };
+
+// Launch with programmatic stream serialisation (see pdl_wait, common.cuh):
+// the kernel's CTAs may become resident once every CTA of the previous kernel
+// has started, and run their table loads under its tail.  The kernel must call
+// pdl_wait.  Launches of more than kPdlMaxThreads (eight times the threads the
+// SMs hold) go out serialised: their tails are a small part of them, and early
+// CTAs cost more than they hide.  Measured at N = 2^16, L = 30, limit at 0 / 2 / 4 /
+// 8 / 16 / no limit: one HMult 306 / 279 / 275 / 266 / 266 / 266 us, bootstrap 24.1 /
+// 23.05 / 22.71 / 22.75 / 22.78 / 23.09 ms, 21 pairs at uneven levels 6.57 / 6.53 /
+// 6.51 / 6.49 / 6.49 / 6.49 ms; a batch of 32 HMults is 1-5% slower without a limit.
+constexpr size_t kPdlMaxThreads = (size_t)8 * 148 * 2048;
+template <class... P, class... A>
+inline void launch_pdl(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = g;
+    cfg.blockDim = b;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = (size_t)g.x * g.y * g.z * b.x * b.y * b.z <= kPdlMaxThreads ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
 
 // process-wide count of kernels launched by this library
 uint64_t launch_count();

@@ -33,6 +33,8 @@ __device__ __forceinline__ uint32_t automorph_slot(int logN, uint32_t k, uint32_
 // for every batch element (blockIdx.z)
 // ---------------------------------------------------------------------------
 __global__ void k_tensor(const __grid_constant__ DevCtx ctx, const __grid_constant__ TensorArgs args) {
+    pdl_trigger();
+    pdl_wait();
     const int limb = blockIdx.y, bi = blockIdx.z;
     const PrimeConst pc = ctx.pc[limb];
     const size_t i = ((size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2);
@@ -84,7 +86,7 @@ __global__ void k_tensor(const __grid_constant__ DevCtx ctx, const __grid_consta
 void launch_tensor(const DevCtx& ctx, int n, int nb, const TensorArgs& args, cudaStream_t st) {
     dim3 g(ctx.N / 256, n, nb);
     count_launches(1);
-    k_tensor<<<g, 128, 0, st>>>(ctx, args);
+    launch_pdl(k_tensor, g, 128, 0, st, ctx, args);
 }
 
 // ---------------------------------------------------------------------------
@@ -120,6 +122,8 @@ __global__ void __launch_bounds__(kConvThreads) k_modup_conv(const __grid_consta
                                                              const uint64_t* __restrict__ xt,
                                                              uint64_t* __restrict__ dig, size_t dig_stride,
                                                              size_t bstride) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ uint64_t sM[MAXIN][kConvTargets];
     __shared__ PrimeConst sP[kConvTargets];
     const int ndig = level / ctx.alpha + 1;
@@ -183,6 +187,8 @@ __global__ void __launch_bounds__(kConvThreads) k_modup_conv_c1(const __grid_con
                                                                 const uint64_t* __restrict__ xt,
                                                                 uint64_t* __restrict__ dig, size_t dig_stride,
                                                                 size_t bstride) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ uint64_t sM[MAXIN][kConvTargets];
     __shared__ PrimeConst sP[kConvTargets];
     const int ndig = level / ctx.alpha + 1;
@@ -248,11 +254,11 @@ void launch_modup_conv(const DevCtx& ctx, int level, int nb, const uint64_t* xt,
     const dim3 g1(ctx.N / kConvThreads, g.y, g.z);
 #define FIDES_MODUP(M)                                                                                       \
     if (ctx.conv_variant == 2)                                                                              \
-        k_modup_conv_c1<M><<<g1, kConvThreads, 0, st>>>(ctx, level, xt, dig, dig_stride, bstride);          \
+        launch_pdl(k_modup_conv_c1<M>, g1, kConvThreads, 0, st, ctx, level, xt, dig, dig_stride, bstride);          \
     else if (ctx.conv_variant == 1)                                                                         \
-        k_modup_conv<M, AccSplit><<<g, kConvThreads, 0, st>>>(ctx, level, xt, dig, dig_stride, bstride);    \
+        launch_pdl(k_modup_conv<M, AccSplit>, g, kConvThreads, 0, st, ctx, level, xt, dig, dig_stride, bstride);    \
     else                                                                                                    \
-        k_modup_conv<M, Acc128><<<g, kConvThreads, 0, st>>>(ctx, level, xt, dig, dig_stride, bstride);
+        launch_pdl(k_modup_conv<M, Acc128>, g, kConvThreads, 0, st, ctx, level, xt, dig, dig_stride, bstride);
     if (ctx.alpha <= 4) {
         FIDES_MODUP(4)
     } else if (ctx.alpha <= 8) {
@@ -297,6 +303,8 @@ constexpr bool kIsSplitAcc<AccSplit> = true;
 template <int VEC, class ACC, bool FPK, bool GRP = false, bool SEED = false>
 __global__ void __launch_bounds__(256, SEED ? (FPK ? 5 : (kIsSplitAcc<ACC> ? 0 : 6)) : 0)
     k_ks_inner(const __grid_constant__ DevCtx ctx, int level, int nb, const __grid_constant__ KsArgs args) {
+    pdl_trigger();
+    pdl_wait();
     const int n = level + 1;
     const int m = blockIdx.y;
     const int bi = blockIdx.x % nb;
@@ -479,9 +487,9 @@ template <int VEC, class ACC, bool FPK, bool GRP>
 static void ks_inner_go(const DevCtx& ctx, int level, int nb, const KsArgs& args, bool seeded, dim3 g,
                         cudaStream_t st) {
     if (seeded)
-        k_ks_inner<VEC, ACC, FPK, GRP, true><<<g, 256, 0, st>>>(ctx, level, nb, args);
+        launch_pdl(k_ks_inner<VEC, ACC, FPK, GRP, true>, g, 256, 0, st, ctx, level, nb, args);
     else
-        k_ks_inner<VEC, ACC, FPK, GRP, false><<<g, 256, 0, st>>>(ctx, level, nb, args);
+        launch_pdl(k_ks_inner<VEC, ACC, FPK, GRP, false>, g, 256, 0, st, ctx, level, nb, args);
 }
 
 void launch_ks_inner(const DevCtx& ctx, int level, int nb, const KsArgs& args, bool plain, cudaStream_t st) {
@@ -526,6 +534,8 @@ void launch_ks_inner(const DevCtx& ctx, int level, int nb, const KsArgs& args, b
 template <int MAXIN, class ACC>
 __global__ void __launch_bounds__(kConvThreads) k_moddown_conv(const __grid_constant__ DevCtx ctx, int level,
                                                                const __grid_constant__ MdArgs args) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ uint64_t sM[MAXIN][kConvTargets];
     __shared__ PrimeConst sP[kConvTargets];
     __shared__ ulonglong2 sPinv[kConvTargets];
@@ -619,9 +629,9 @@ void launch_moddown_conv(const DevCtx& ctx, int level, int nb, const MdArgs& a, 
     count_launches(1);
 #define FIDES_MODDOWN(M)                                                      \
     if (ctx.conv_variant == 1)                                                \
-        k_moddown_conv<M, AccSplit><<<g, kConvThreads, 0, st>>>(ctx, level, a); \
+        launch_pdl(k_moddown_conv<M, AccSplit>, g, kConvThreads, 0, st, ctx, level, a); \
     else                                                                      \
-        k_moddown_conv<M, Acc128><<<g, kConvThreads, 0, st>>>(ctx, level, a);
+        launch_pdl(k_moddown_conv<M, Acc128>, g, kConvThreads, 0, st, ctx, level, a);
     if (ctx.K <= 4) {
         FIDES_MODDOWN(4)
     } else if (ctx.K <= 8) {
@@ -640,6 +650,8 @@ void launch_moddown_conv(const DevCtx& ctx, int level, int nb, const MdArgs& a, 
 template <int OP>
 __global__ void k_elementwise(const __grid_constant__ DevCtx ctx, int q0, const uint64_t* __restrict__ a,
                               const uint64_t* __restrict__ b, uint64_t* __restrict__ out) {
+    pdl_trigger();
+    pdl_wait();
     const int limb = blockIdx.y;
     const PrimeConst pc = ctx.pc[q0 + limb];
     const size_t i = (size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2;
@@ -671,11 +683,11 @@ void launch_elementwise(const DevCtx& ctx, int op, int n, int q0, const uint64_t
     if (n <= 0) return;
     dim3 g(ctx.N / 256, n);
     switch (op) {
-        case EW_ADD: count_launches(1); k_elementwise<EW_ADD><<<g, 128, 0, st>>>(ctx, q0, a, b, out); break;
-        case EW_SUB: count_launches(1); k_elementwise<EW_SUB><<<g, 128, 0, st>>>(ctx, q0, a, b, out); break;
-        case EW_NEG: count_launches(1); k_elementwise<EW_NEG><<<g, 128, 0, st>>>(ctx, q0, a, b, out); break;
-        case EW_MUL: count_launches(1); k_elementwise<EW_MUL><<<g, 128, 0, st>>>(ctx, q0, a, b, out); break;
-        default: count_launches(1); k_elementwise<EW_COPY><<<g, 128, 0, st>>>(ctx, q0, a, b, out); break;
+        case EW_ADD: count_launches(1); launch_pdl(k_elementwise<EW_ADD>, g, 128, 0, st, ctx, q0, a, b, out); break;
+        case EW_SUB: count_launches(1); launch_pdl(k_elementwise<EW_SUB>, g, 128, 0, st, ctx, q0, a, b, out); break;
+        case EW_NEG: count_launches(1); launch_pdl(k_elementwise<EW_NEG>, g, 128, 0, st, ctx, q0, a, b, out); break;
+        case EW_MUL: count_launches(1); launch_pdl(k_elementwise<EW_MUL>, g, 128, 0, st, ctx, q0, a, b, out); break;
+        default: count_launches(1); launch_pdl(k_elementwise<EW_COPY>, g, 128, 0, st, ctx, q0, a, b, out); break;
     }
 }
 
@@ -684,6 +696,8 @@ void launch_elementwise(const DevCtx& ctx, int op, int n, int q0, const uint64_t
 // limbs, at bstride) are added into element start[u].  Two coefficients per
 // thread.
 __global__ void k_ext_sum(const __grid_constant__ DevCtx ctx, const __grid_constant__ ExtSumArgs a) {
+    pdl_trigger();
+    pdl_wait();
     const int limb = blockIdx.y, u = blockIdx.z;
     const int j = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (j >= ctx.N) return;
@@ -705,12 +719,14 @@ __global__ void k_ext_sum(const __grid_constant__ DevCtx ctx, const __grid_const
 void launch_ext_sum(const DevCtx& ctx, const ExtSumArgs& a, cudaStream_t st) {
     if (a.nout <= 0) return;
     count_launches(1);
-    k_ext_sum<<<dim3((ctx.N + 511) / 512, a.n + ctx.K, a.nout), 256, 0, st>>>(ctx, a);
+    launch_pdl(k_ext_sum, dim3((ctx.N + 511) / 512, a.n + ctx.K, a.nout), 256, 0, st, ctx, a);
 }
 
 __global__ void k_scalar_mac(const __grid_constant__ DevCtx ctx, const uint64_t* __restrict__ a,
                              const uint64_t* __restrict__ cj, const uint64_t* __restrict__ b,
                              uint64_t* __restrict__ out) {
+    pdl_trigger();
+    pdl_wait();
     const int limb = blockIdx.y;
     const PrimeConst pc = ctx.pc[limb];
     const ulonglong2 c = __ldg(reinterpret_cast<const ulonglong2*>(cj) + limb);
@@ -732,11 +748,13 @@ void launch_scalar_mac(const DevCtx& ctx, int n, const uint64_t* a, const uint64
     if (n <= 0) return;
     dim3 g(ctx.N / 256, n);
     count_launches(1);
-    k_scalar_mac<<<g, 128, 0, st>>>(ctx, a, cj, b, out);
+    launch_pdl(k_scalar_mac, g, 128, 0, st, ctx, a, cj, b, out);
 }
 
 __global__ void k_scalar_add(const __grid_constant__ DevCtx ctx, const uint64_t* __restrict__ a,
                              const uint64_t* __restrict__ cj, uint64_t* __restrict__ out) {
+    pdl_trigger();
+    pdl_wait();
     const int limb = blockIdx.y;
     const PrimeConst pc = ctx.pc[limb];
     const uint64_t c = __ldg(cj + limb);
@@ -753,7 +771,7 @@ void launch_scalar_add(const DevCtx& ctx, int n, const uint64_t* a, const uint64
     if (n <= 0) return;
     dim3 g(ctx.N / 256, n);
     count_launches(1);
-    k_scalar_add<<<g, 128, 0, st>>>(ctx, a, cj, out);
+    launch_pdl(k_scalar_add, g, 128, 0, st, ctx, a, cj, out);
 }
 
 // Plaintext dot product: each thread owns two coefficients of both halves,
@@ -762,6 +780,8 @@ void launch_scalar_add(const DevCtx& ctx, int n, const uint64_t* a, const uint64
 // the accumulators are folded back to one residue every 15 terms.
 // Role in the reference: dotProductPt_ (CKKS/ElemenwiseBatchKernels.cu:651).
 __global__ void k_dot_pt(const __grid_constant__ DevCtx ctx, const __grid_constant__ DotArgs args) {
+    pdl_trigger();
+    pdl_wait();
     const int limb = blockIdx.y;
     const PrimeConst pc = ctx.pc[limb];
     const size_t i = (size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2;
@@ -805,12 +825,14 @@ void launch_dot_pt(const DevCtx& ctx, int nlimbs, const DotArgs& args, cudaStrea
     if (nlimbs <= 0 || args.n <= 0 || args.n > kMaxBatch) return;
     dim3 g(ctx.N / 256, nlimbs);
     count_launches(1);
-    k_dot_pt<<<g, 128, 0, st>>>(ctx, args);
+    launch_pdl(k_dot_pt, g, 128, 0, st, ctx, args);
 }
 
 // Integer linear combination (leaf sums of polynomial evaluation, integer
 // scalar products): each thread owns two coefficients of both components.
 __global__ void k_lincomb(const __grid_constant__ DevCtx ctx, const __grid_constant__ LinArgs args) {
+    pdl_trigger();
+    pdl_wait();
     const int limb = blockIdx.y;
     const PrimeConst pc = ctx.pc[args.q0 + limb];
     const size_t i = (size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2;
@@ -837,7 +859,7 @@ void launch_lincomb(const DevCtx& ctx, int nlimbs, const LinArgs& args, cudaStre
     if (nlimbs <= 0 || nlimbs > kMaxLinLimbs || args.n < 0 || args.n > kMaxLin) return;
     dim3 g(ctx.N / 256, nlimbs);
     count_launches(1);
-    k_lincomb<<<g, 128, 0, st>>>(ctx, args);
+    launch_pdl(k_lincomb, g, 128, 0, st, ctx, args);
 }
 
 // X^k in evaluation form: slot i of prime j holds psi_j^e, e = (2 brev(i) + 1) k
@@ -846,6 +868,8 @@ void launch_lincomb(const DevCtx& ctx, int nlimbs, const LinArgs& args, cudaStre
 __global__ void k_mult_monomial(const __grid_constant__ DevCtx ctx, const uint64_t* __restrict__ in0,
                                 const uint64_t* __restrict__ in1, uint64_t* __restrict__ out0,
                                 uint64_t* __restrict__ out1, uint32_t k) {
+    pdl_trigger();
+    pdl_wait();
     const int limb = blockIdx.y;
     const uint64_t* in = blockIdx.z ? in1 : in0;
     uint64_t* out = blockIdx.z ? out1 : out0;
@@ -866,11 +890,13 @@ void launch_mult_monomial(const DevCtx& ctx, int nlimbs, const uint64_t* in0, co
     if (nlimbs <= 0) return;
     dim3 g(ctx.N / 256, nlimbs, 2);
     count_launches(1);
-    k_mult_monomial<<<g, 256, 0, st>>>(ctx, in0, in1, out0, out1, k);
+    launch_pdl(k_mult_monomial, g, 256, 0, st, ctx, in0, in1, out0, out1, k);
 }
 
 __global__ void k_automorph(const __grid_constant__ DevCtx ctx, const uint64_t* __restrict__ in,
                             uint64_t* __restrict__ out, uint32_t galois_inv) {
+    pdl_trigger();
+    pdl_wait();
     const size_t base = (size_t)blockIdx.y * ctx.N;
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     out[base + j] = in[base + automorph_slot(ctx.logN, galois_inv, j)];
@@ -881,7 +907,7 @@ void launch_automorph(const DevCtx& ctx, int nlimbs, const uint64_t* in, uint64_
     if (nlimbs <= 0) return;
     dim3 g(ctx.N / 256, nlimbs);
     count_launches(1);
-    k_automorph<<<g, 256, 0, st>>>(ctx, in, out, galois_inv);
+    launch_pdl(k_automorph, g, 256, 0, st, ctx, in, out, galois_inv);
 }
 
 }  // namespace fides

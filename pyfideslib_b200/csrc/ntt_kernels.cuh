@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
     __shared__ __align__(16) uint64_t sm[LR > 4 ? G::R * TC : 1];
     __shared__ ulonglong2 tws[G::R];
 
+    pdl_trigger();
     const LimbRef lr = resolve_limb(map, blockIdx.z, blockIdx.y, ctx.N, ctx.L);
     const PrimeConst pc = ctx.pc[lr.prime];
     const bool fp = FP && pc.p < kFpPrimeBound;
@@ -283,6 +284,7 @@ __global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
 
     const int c = threadIdx.x % TC, th = threadIdx.x / TC;
     const int col = blockIdx.x * TC + c;
+    pdl_wait();
     uint64_t x[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) x[k] = lr.in[(size_t)(th + (k << (LR - 4))) * C + col];
@@ -431,6 +433,7 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
     __shared__ __align__(16) uint64_t sm[G::W * G::SW];
     __shared__ ulonglong2 s_twa[G::W * G::TW];
 
+    pdl_trigger();
     const LimbRef lr = resolve_limb(map, blockIdx.z, blockIdx.y, ctx.N, ctx.L);
     const PrimeConst pc = ctx.pc[lr.prime];
     const bool fp = FP && pc.p < kFpPrimeBound;
@@ -445,6 +448,7 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
     stage_row_tw<LR, LC>(s_tw, twg, row0, lane);
     RowFwd<LR, LC, FP> rf;
     if (fp) rf.load_d(twg, row0 + rl, th);
+    pdl_wait();
     const uint64_t* src = lr.out + base + rl * G::C;
     uint64_t x[16];
 #pragma unroll
@@ -560,6 +564,7 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
     using G = RowGeo<LR, LC>;
     extern __shared__ __align__(16) uint64_t ks_sm[];  // per warp: twiddles, then one tile per digit needing rows
 
+    pdl_trigger();
     const int level = a.level, n = level + 1;
     const int m = a.m0 + (int)blockIdx.z;
     const size_t boff = (size_t)blockIdx.y * a.bstride;
@@ -589,6 +594,7 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
         prefetch_l2(a.kb + d * kstride + limb_off + lane * 16);
         prefetch_l2(a.ka + d * kstride + limb_off + lane * 16);
     }
+    pdl_wait();
     if (d_own >= 0) prefetch_l2(a.own + boff + limb_off + lane * 16);
     stage_wait();
     __syncwarp(G::MASK);
@@ -704,6 +710,7 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
     __shared__ __align__(16) uint64_t sm[G::W * G::SW];
     __shared__ ulonglong2 s_twa[G::W * G::TW];
 
+    pdl_trigger();
     const LimbRef lr = resolve_limb(map, blockIdx.z, blockIdx.y, ctx.N, ctx.L);
     const PrimeConst pc = ctx.pc[lr.prime];
     const bool fp = FP && pc.p < kFpPrimeBound;
@@ -725,6 +732,7 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
             D[kb] = ldg2(twg, ((size_t)(G::R + row) << (LC - 1 - kb)) + ((size_t)th << (3 - kb)));
     }
     const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
+    pdl_wait();
     uint64_t x[16];
     {
         // all 16 words of the lane are loaded before any is used, so the
@@ -825,6 +833,7 @@ __global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
     __shared__ __align__(16) uint64_t sm[LR > 4 ? G::R * TC : 1];
     __shared__ ulonglong2 tws[G::R];
 
+    pdl_trigger();
     const LimbRef lr = resolve_limb(map, blockIdx.z, blockIdx.y, ctx.N, ctx.L);
     const PrimeConst pc = ctx.pc[lr.prime];
     const bool fp = FP && pc.p < kFpPrimeBound;
@@ -836,6 +845,7 @@ __global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
     const int c = threadIdx.x % TC, th = threadIdx.x / TC;
     const int col = blockIdx.x * TC + c;
     const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
+    pdl_wait();
     uint64_t x[16];
     if constexpr (LR > 4) {
 #pragma unroll
@@ -898,24 +908,24 @@ struct NttN {
 
     static void fwd_cols(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
         if (ntt_fwd_is_fp(ctx.ntt_variant))
-            k_ntt_fwd_cols<LR, LC, true><<<gcols(map), CG::NT, 0, st>>>(ctx, map);
+            launch_pdl(k_ntt_fwd_cols<LR, LC, true>, gcols(map), CG::NT, 0, st, ctx, map);
         else
-            k_ntt_fwd_cols<LR, LC, false><<<gcols(map), CG::NT, 0, st>>>(ctx, map);
+            launch_pdl(k_ntt_fwd_cols<LR, LC, false>, gcols(map), CG::NT, 0, st, ctx, map);
     }
     static void fwd(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
         fwd_cols(ctx, map, st);
         if (ntt_fwd_is_fp(ctx.ntt_variant))
-            k_ntt_fwd_rows<LR, LC, true><<<grows(map), RG::NT, 0, st>>>(ctx, map);
+            launch_pdl(k_ntt_fwd_rows<LR, LC, true>, grows(map), RG::NT, 0, st, ctx, map);
         else
-            k_ntt_fwd_rows<LR, LC, false><<<grows(map), RG::NT, 0, st>>>(ctx, map);
+            launch_pdl(k_ntt_fwd_rows<LR, LC, false>, grows(map), RG::NT, 0, st, ctx, map);
     }
     static void inv(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
         if (ntt_inv_is_fp(ctx.intt_variant)) {
-            k_ntt_inv_rows<LR, LC, true><<<grows(map), RG::NT, 0, st>>>(ctx, map);
-            k_ntt_inv_cols<LR, LC, true><<<gcols(map), CG::NT, 0, st>>>(ctx, map);
+            launch_pdl(k_ntt_inv_rows<LR, LC, true>, grows(map), RG::NT, 0, st, ctx, map);
+            launch_pdl(k_ntt_inv_cols<LR, LC, true>, gcols(map), CG::NT, 0, st, ctx, map);
         } else {
-            k_ntt_inv_rows<LR, LC, false><<<grows(map), RG::NT, 0, st>>>(ctx, map);
-            k_ntt_inv_cols<LR, LC, false><<<gcols(map), CG::NT, 0, st>>>(ctx, map);
+            launch_pdl(k_ntt_inv_rows<LR, LC, false>, grows(map), RG::NT, 0, st, ctx, map);
+            launch_pdl(k_ntt_inv_cols<LR, LC, false>, gcols(map), CG::NT, 0, st, ctx, map);
         }
     }
 
@@ -934,11 +944,11 @@ struct NttN {
             KsFuseArgs sp = a;
             sp.m0 = n;
             count_launches(1);
-            k_ntt_fwd_rows_ks<LR, LC, FP, 6><<<grid(n), RG::NT, bytes(nd - 1), st>>>(ctx, q, nd - 1);
-            k_ntt_fwd_rows_ks<LR, LC, FP, 4><<<grid(ctx.K), RG::NT, bytes(nd), st>>>(ctx, sp, nd);
+            launch_pdl(k_ntt_fwd_rows_ks<LR, LC, FP, 6>, grid(n), RG::NT, bytes(nd - 1), st, ctx, q, nd - 1);
+            launch_pdl(k_ntt_fwd_rows_ks<LR, LC, FP, 4>, grid(ctx.K), RG::NT, bytes(nd), st, ctx, sp, nd);
             return;
         }
-        k_ntt_fwd_rows_ks<LR, LC, FP, 4><<<grid(n + ctx.K), RG::NT, bytes(nd), st>>>(ctx, q, nd);
+        launch_pdl(k_ntt_fwd_rows_ks<LR, LC, FP, 4>, grid(n + ctx.K), RG::NT, bytes(nd), st, ctx, q, nd);
     }
     static void rows_ks(const DevCtx& ctx, const KsFuseArgs& a, int nb, cudaStream_t st) {
         if (ntt_fwd_is_fp(ctx.ntt_variant))
