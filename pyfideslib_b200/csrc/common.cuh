@@ -73,7 +73,8 @@ struct DevCtx {
     const uint64_t* md_pinv;     // [L][2]       P^-1 mod q_j
     const uint64_t* md_pmod;     // [L][2]       P mod q_j
     const uint64_t* rs_qinv;     // [L][L][2]    q_l^-1 mod q_j (row l, column j < l)
-    const double* md_pinvf;      // [L][2]       the same two as doubles: the residue centred in (-q_j/2, q_j/2]
+    const double* md_pmodf;      // [L][2]       P mod q_j the same way (below)
+    const double* md_pinvf;      // [L][2]       the two inverses as doubles: the residue centred in (-q_j/2, q_j/2]
     const double* rs_qinvf;      // [L][L][2]    and its quotient by q_j (primes below 2^50, else 0)
     const uint8_t* tc_btab;      // tensor-core conversions: byte matrices B per (level, digit) and
     const uint64_t* tc_boff;     //   per (level, fused) for ModDown, and their byte offsets (or null)

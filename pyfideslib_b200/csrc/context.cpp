@@ -443,7 +443,7 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
         }
 
     // the same inverses as centred doubles with their quotients (FP64 epilogues)
-    std::vector<double> md_pinvf((size_t)L * 2, 0.0), rs_qinvf((size_t)L * L * 2, 0.0);
+    std::vector<double> md_pmodf((size_t)L * 2, 0.0), md_pinvf((size_t)L * 2, 0.0), rs_qinvf((size_t)L * L * 2, 0.0);
     auto centred = [&](uint64_t v, uint64_t pr, double* out) {
         if (pr >= kFpPrimeBound) return;
         out[0] = v > (pr >> 1) ? -(double)(pr - v) : (double)v;
@@ -451,6 +451,7 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
     };
     for (int j = 0; j < L; ++j) {
         centred(md_pinv[2 * j], P(j), &md_pinvf[2 * j]);
+        centred(md_pmod[2 * j], P(j), &md_pmodf[2 * j]);
         for (int l = j + 1; l < L; ++l)
             centred(rs_qinv[((size_t)l * L + j) * 2], P(j), &rs_qinvf[((size_t)l * L + j) * 2]);
     }
@@ -489,6 +490,7 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
     size_t i_dp = add(md_pinv.data(), md_pinv.size() * 8);
     size_t i_dq = add(md_pmod.data(), md_pmod.size() * 8);
     size_t i_rq = add(rs_qinv.data(), rs_qinv.size() * 8);
+    size_t i_dqf = add(md_pmodf.data(), md_pmodf.size() * 8);
     size_t i_dpf = add(md_pinvf.data(), md_pinvf.size() * 8);
     size_t i_rqf = add(rs_qinvf.data(), rs_qinvf.size() * 8);
     const uint64_t zero_word = 0;
@@ -521,6 +523,7 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
     d.md_pinv = (const uint64_t*)(base + parts[i_dp].off);
     d.md_pmod = (const uint64_t*)(base + parts[i_dq].off);
     d.rs_qinv = (const uint64_t*)(base + parts[i_rq].off);
+    d.md_pmodf = (const double*)(base + parts[i_dqf].off);
     d.md_pinvf = (const double*)(base + parts[i_dpf].off);
     d.rs_qinvf = (const double*)(base + parts[i_rqf].off);
     d.err = (uint32_t*)(base + parts[i_err].off);

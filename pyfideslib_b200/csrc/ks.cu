@@ -362,10 +362,10 @@ __global__ void __launch_bounds__(256, SEED ? (FPK ? 5 : (kIsSplitAcc<ACC> ? 0 :
                 }
             }
             ulonglong2 ob, oa;
-            ob.x = fp_to_u(fp_center(sb0, p, pinv), p, pinv);
-            ob.y = fp_to_u(fp_center(sb1, p, pinv), p, pinv);
-            oa.x = fp_to_u(fp_center(sa0, p, pinv), p, pinv);
-            oa.y = fp_to_u(fp_center(sa1, p, pinv), p, pinv);
+            ob.x = fp_sum_to_u(sb0, p, pinv);
+            ob.y = fp_sum_to_u(sb1, p, pinv);
+            oa.x = fp_sum_to_u(sa0, p, pinv);
+            oa.y = fp_sum_to_u(sa1, p, pinv);
             *reinterpret_cast<ulonglong2*>(xb + j) = ob;
             *reinterpret_cast<ulonglong2*>(xa + j) = oa;
             return;
@@ -402,47 +402,63 @@ __global__ void __launch_bounds__(256, SEED ? (FPK ? 5 : (kIsSplitAcc<ACC> ? 0 :
     } else {
         // rotation: outputs j, j+1 gather the digit values (and c0) at the
         // automorphism's source slots; the key is stored permuted (entry j is
-        // the one that pairs with output j), so its loads stay vectorised
+        // the one that pairs with output j), so its loads stay vectorised.
+        // Slots 2i and 2i+1 belong to exponents e and e + N, and g (e + N) =
+        // g e + N mod 2N for odd g: the sources of an adjacent pair are an
+        // adjacent pair, possibly swapped, and are read as one 16-byte word.
+        // (With one 8-byte gather per output and integer products by P this
+        // branch took 851 us for 32 rotations of 20 limbs at N = 2^16, 70% of
+        // the issue slots busy.)
         const size_t j = ((size_t)bx * blockDim.x + threadIdx.x) * 2;
         const uint32_t g = args.galois[bi];
         const uint32_t s0 = g ? automorph_slot(ctx.logN, g, (uint32_t)j) : (uint32_t)j;
-        const uint32_t s1 = g ? automorph_slot(ctx.logN, g, (uint32_t)j + 1) : (uint32_t)j + 1;
+        const bool swap = s0 & 1;
+        const size_t sp = s0 & ~1u;
+        auto gather = [&](const uint64_t* src) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src + sp);
+            return swap ? make_ulonglong2(v.y, v.x) : v;
+        };
         const size_t koff = (size_t)t * ctx.N + j;
         const uint64_t* c0 = args.c0[bi];
+        auto key_a = [&](int d) {
+            ulonglong2 a;
+            if (!SEED || ka) {
+                a = *reinterpret_cast<const ulonglong2*>(ka + d * kstride + koff);
+            } else {
+                a.x = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j, pc.p);
+                a.y = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j + 1, pc.p);
+            }
+            return a;
+        };
         if constexpr (FPK) {
-            // up to 6 digits: |sum| <= 6 * 0.875p + p (the P c0 term) < 2^53
+            // up to 6 digits: |sum| <= 6 * 0.875p + 0.54p (the P c0 term) < 8p
             if (pc.p < kFpPrimeBound && nd <= 6) {
                 const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
                 double sb0 = 0, sb1 = 0, sa0 = 0, sa1 = 0;
+                if (c0 && m < n) {
+                    const double2 pm = __ldg(reinterpret_cast<const double2*>(ctx.md_pmodf) + t);
+                    const ulonglong2 c = gather(c0 + (size_t)m * ctx.N);
+                    sb0 = fp_mulw(as_f64(fp_from_u(c.x)), pm.x, pm.y, p);
+                    sb1 = fp_mulw(as_f64(fp_from_u(c.y)), pm.x, pm.y, p);
+                }
 #pragma unroll
                 for (int d = 0; d < 6; ++d) {
                     if (d < nd) {
-                        const double x0 = as_f64(fp_from_u(srcs[d][s0])), x1 = as_f64(fp_from_u(srcs[d][s1]));
+                        const ulonglong2 x = gather(srcs[d]);
                         const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(kb + d * kstride + koff);
-                        ulonglong2 a;
-                        if (!SEED || ka) {
-                            a = *reinterpret_cast<const ulonglong2*>(ka + d * kstride + koff);
-                        } else {
-                            a.x = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j, pc.p);
-                            a.y = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j + 1, pc.p);
-                        }
+                        const ulonglong2 a = key_a(d);
+                        const double x0 = as_f64(fp_from_u(x.x)), x1 = as_f64(fp_from_u(x.y));
                         sb0 = __dadd_rn(sb0, fp_mulmod(x0, as_f64(fp_from_u(b.x)), p, pinv));
                         sb1 = __dadd_rn(sb1, fp_mulmod(x1, as_f64(fp_from_u(b.y)), p, pinv));
                         sa0 = __dadd_rn(sa0, fp_mulmod(x0, as_f64(fp_from_u(a.x)), p, pinv));
                         sa1 = __dadd_rn(sa1, fp_mulmod(x1, as_f64(fp_from_u(a.y)), p, pinv));
                     }
                 }
-                if (c0 && m < n) {
-                    const ulonglong2 pm = __ldg(reinterpret_cast<const ulonglong2*>(ctx.md_pmod) + t);
-                    const uint64_t* cm = c0 + (size_t)m * ctx.N;
-                    sb0 = __dadd_rn(sb0, as_f64(fp_from_u(mul_shoup(cm[s0], pm.x, pm.y, pc.p))));
-                    sb1 = __dadd_rn(sb1, as_f64(fp_from_u(mul_shoup(cm[s1], pm.x, pm.y, pc.p))));
-                }
                 ulonglong2 ob, oa;
-                ob.x = fp_to_u(fp_center(sb0, p, pinv), p, pinv);
-                ob.y = fp_to_u(fp_center(sb1, p, pinv), p, pinv);
-                oa.x = fp_to_u(fp_center(sa0, p, pinv), p, pinv);
-                oa.y = fp_to_u(fp_center(sa1, p, pinv), p, pinv);
+                ob.x = fp_sum_to_u(sb0, p, pinv);
+                ob.y = fp_sum_to_u(sb1, p, pinv);
+                oa.x = fp_sum_to_u(sa0, p, pinv);
+                oa.y = fp_sum_to_u(sa1, p, pinv);
                 *reinterpret_cast<ulonglong2*>(xb + j) = ob;
                 *reinterpret_cast<ulonglong2*>(xa + j) = oa;
                 return;
@@ -452,26 +468,20 @@ __global__ void __launch_bounds__(256, SEED ? (FPK ? 5 : (kIsSplitAcc<ACC> ? 0 :
 #pragma unroll
         for (int d = 0; d < 8; ++d) {
             if (d < nd) {
-                const uint64_t x0 = srcs[d][s0], x1 = srcs[d][s1];
+                const ulonglong2 x = gather(srcs[d]);
                 const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(kb + d * kstride + koff);
-                ulonglong2 a;
-                if (!SEED || ka) {
-                    a = *reinterpret_cast<const ulonglong2*>(ka + d * kstride + koff);
-                } else {
-                    a.x = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j, pc.p);
-                    a.y = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j + 1, pc.p);
-                }
-                sb0.mac(x0, b.x);
-                sb1.mac(x1, b.y);
-                sa0.mac(x0, a.x);
-                sa1.mac(x1, a.y);
+                const ulonglong2 a = key_a(d);
+                sb0.mac(x.x, b.x);
+                sb1.mac(x.y, b.y);
+                sa0.mac(x.x, a.x);
+                sa1.mac(x.y, a.y);
             }
         }
         if (c0 && m < n) {
             const ulonglong2 pm = __ldg(reinterpret_cast<const ulonglong2*>(ctx.md_pmod) + t);
-            const uint64_t* cm = c0 + (size_t)m * ctx.N;
-            sb0.mac(mul_shoup(cm[s0], pm.x, pm.y, pc.p), 1);
-            sb1.mac(mul_shoup(cm[s1], pm.x, pm.y, pc.p), 1);
+            const ulonglong2 c = gather(c0 + (size_t)m * ctx.N);
+            sb0.mac(mul_shoup(c.x, pm.x, pm.y, pc.p), 1);
+            sb1.mac(mul_shoup(c.y, pm.x, pm.y, pc.p), 1);
         }
         ulonglong2 ob, oa;
         ob.x = sb0.reduce(pc);
