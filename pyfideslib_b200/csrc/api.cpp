@@ -853,8 +853,8 @@ static fides_status binary_op(fides_ctx* c, int op, const fides_ct* a, const fid
     fides_ct tmp;
     fides_status s = ct_reserve(c, &tmp, level);
     if (s != FIDES_OK) return s;
-    launch_elementwise(c->dev, op, n, 0, a->c0(), b ? b->c0() : nullptr, tmp.c0(), c->st);
-    launch_elementwise(c->dev, op, n, 0, a->c1(N), b ? b->c1(N) : nullptr, tmp.c1(N), c->st);
+    const EwArgs e = {{a->c0(), a->c1(N)}, {b ? b->c0() : nullptr, b ? b->c1(N) : nullptr}, {tmp.c0(), tmp.c1(N)}, {op, op}};
+    launch_elementwise2(c->dev, n, 0, e, c->st);
     const double sc = a->scale;
     const int nd = a->noise_deg, sl = std::max(a->slots, b ? b->slots : 0);
     commit(c, out, tmp);
@@ -888,8 +888,8 @@ fides_status fides_add_pt(fides_ctx* c, const fides_ct* a, const fides_pt* p, fi
     fides_ct tmp;
     fides_status s = ct_reserve(c, &tmp, level);
     if (s != FIDES_OK) return s;
-    launch_elementwise(c->dev, EW_ADD, n, 0, a->c0(), p->m, tmp.c0(), c->st);
-    launch_elementwise(c->dev, EW_COPY, n, 0, a->c1(N), nullptr, tmp.c1(N), c->st);
+    const EwArgs e = {{a->c0(), a->c1(N)}, {p->m, nullptr}, {tmp.c0(), tmp.c1(N)}, {EW_ADD, EW_COPY}};
+    launch_elementwise2(c->dev, n, 0, e, c->st);
     const double sc = a->scale;
     const int nd = a->noise_deg, sl = std::max(a->slots, p->slots);
     commit(c, out, tmp);
@@ -907,8 +907,8 @@ fides_status fides_mult_pt(fides_ctx* c, const fides_ct* a, const fides_pt* p, f
     fides_ct tmp;
     fides_status s = ct_reserve(c, &tmp, level);
     if (s != FIDES_OK) return s;
-    launch_elementwise(c->dev, EW_MUL, n, 0, a->c0(), p->m, tmp.c0(), c->st);
-    launch_elementwise(c->dev, EW_MUL, n, 0, a->c1(N), p->m, tmp.c1(N), c->st);
+    const EwArgs e = {{a->c0(), a->c1(N)}, {p->m, p->m}, {tmp.c0(), tmp.c1(N)}, {EW_MUL, EW_MUL}};
+    launch_elementwise2(c->dev, n, 0, e, c->st);
     const double sc = a->scale * p->scale;
     const int nd = a->noise_deg + p->noise_deg, sl = std::max(a->slots, p->slots);
     commit(c, out, tmp);
@@ -921,22 +921,38 @@ fides_status fides_mult_pt(fides_ctx* c, const fides_ct* a, const fides_pt* p, f
     return st;
 }
 
+}  // extern "C"
+
+// out = a times the per-limb constants k (value, Shoup companion) or, without
+// mul, a plus them; both components per launch
+static void ct_scalar(fides_ctx* c, const fides_ct* a, bool mul, const std::vector<uint64_t>& k, fides_ct& tmp) {
+    const int n = a->level + 1, N = c->N;
+    for (int j0 = 0; j0 < n; j0 += kMaxLinLimbs) {
+        const int nl = std::min(kMaxLinLimbs, n - j0);
+        const size_t off = (size_t)j0 * N;
+        CtScalarArgs s{};
+        s.a[0] = a->c0() + off;
+        s.a[1] = a->c1(N) + off;
+        s.o[0] = tmp.c0() + off;
+        s.o[1] = tmp.c1(N) + off;
+        s.q0 = j0;
+        memcpy(s.c, k.data() + 2 * j0, sizeof(uint64_t) * 2 * nl);
+        launch_ct_scalar(c->dev, mul, nl, s, c->st);
+    }
+}
+
+extern "C" {
+
 fides_status fides_add_scalar(fides_ctx* c, const fides_ct* a, double v, fides_ct* out) {
     if (!c || !valid_ct(c, a) || !out) return FIDES_BAD_ARG;
     Guard g(c);
-    const int n = a->level + 1, N = c->N;
-    std::vector<uint64_t> k(n);
-    for (int j = 0; j < n; ++j) k[j] = round_to_mod((long double)v * a->scale, c->host.prime[j]);
+    const int n = a->level + 1;
+    std::vector<uint64_t> k(2 * n);
+    for (int j = 0; j < n; ++j) k[2 * j] = round_to_mod((long double)v * a->scale, c->host.prime[j]);
     fides_ct tmp;
     fides_status s = ct_reserve(c, &tmp, a->level);
     if (s != FIDES_OK) return s;
-    uint64_t* dk = nullptr;
-    if (cudaMallocAsync((void**)&dk, n * 8, c->st) != cudaSuccess) return set_err(c, FIDES_OOM, "scalar table");
-    cudaMemcpyAsync(dk, k.data(), n * 8, cudaMemcpyHostToDevice, c->st);
-    launch_scalar_add(c->dev, n, a->c0(), dk, tmp.c0(), c->st);
-    launch_elementwise(c->dev, EW_COPY, n, 0, a->c1(N), nullptr, tmp.c1(N), c->st);
-    cudaStreamSynchronize(c->st);
-    cudaFreeAsync(dk, c->st);
+    ct_scalar(c, a, false, k, tmp);
     const fides_ct meta = *a;
     commit(c, out, tmp);
     out->level = meta.level;
@@ -949,7 +965,7 @@ fides_status fides_add_scalar(fides_ctx* c, const fides_ct* a, double v, fides_c
 fides_status fides_mult_scalar(fides_ctx* c, const fides_ct* a, double v, fides_ct* out, int rescale) {
     if (!c || !valid_ct(c, a) || !out) return FIDES_BAD_ARG;
     Guard g(c);
-    const int n = a->level + 1, N = c->N;
+    const int n = a->level + 1;
     const double delta = c->default_scale;
     std::vector<uint64_t> k(2 * n);
     for (int j = 0; j < n; ++j) {
@@ -960,13 +976,7 @@ fides_status fides_mult_scalar(fides_ctx* c, const fides_ct* a, double v, fides_
     fides_ct tmp;
     fides_status s = ct_reserve(c, &tmp, a->level);
     if (s != FIDES_OK) return s;
-    uint64_t* dk = nullptr;
-    if (cudaMallocAsync((void**)&dk, 2 * n * 8, c->st) != cudaSuccess) return set_err(c, FIDES_OOM, "scalar table");
-    cudaMemcpyAsync(dk, k.data(), 2 * n * 8, cudaMemcpyHostToDevice, c->st);
-    launch_scalar_mac(c->dev, n, a->c0(), dk, nullptr, tmp.c0(), c->st);
-    launch_scalar_mac(c->dev, n, a->c1(N), dk, nullptr, tmp.c1(N), c->st);
-    cudaStreamSynchronize(c->st);
-    cudaFreeAsync(dk, c->st);
+    ct_scalar(c, a, true, k, tmp);
     const fides_ct meta = *a;
     commit(c, out, tmp);
     out->level = meta.level;
@@ -1274,8 +1284,8 @@ fides_status giant_rotate_sum(fides_ctx* c, int level, const std::vector<const f
             have_acc[u] = 1;
             return FIDES_OK;
         }
-        launch_elementwise(c->dev, EW_ADD, nl, 0, a->c0(), r->c0(), a->c0(), c->st);
-        launch_elementwise(c->dev, EW_ADD, nl, 0, a->c1(N), r->c1(N), a->c1(N), c->st);
+        const EwArgs e = {{a->c0(), a->c1(N)}, {r->c0(), r->c1(N)}, {a->c0(), a->c1(N)}, {EW_ADD, EW_ADD}};
+        launch_elementwise2(c->dev, nl, 0, e, c->st);
         return FIDES_OK;
     };
     std::vector<int> terms;  // rotations that need a key switch, in owner order
@@ -1449,19 +1459,26 @@ fides_status fides::linear_transform_batch(fides_ctx* c, int nx, const fides_ct*
         for (size_t i = 0; i < inner.size(); ++i) rot.push_back(tmp.make());
         s = fides_rotate_batch(c, (int)inner.size(), inner.data(), gidx.data(), rot.data());
         if (s != FIDES_OK) return s;
-        const size_t bytes = (size_t)nl * c->limb_bytes();
-        for (size_t i = 0; i < rot.size(); ++i) {
-            fides_ct* a = acc[owner[i]];
-            if (!have_acc[owner[i]]) {
-                s = ct_reserve(c, a, level);
-                if (s != FIDES_OK) return s;
-                cudaMemcpyAsync(a->c0(), rot[i]->c0(), bytes, cudaMemcpyDeviceToDevice, c->st);
-                cudaMemcpyAsync(a->c1(N), rot[i]->c1(N), bytes, cudaMemcpyDeviceToDevice, c->st);
-                have_acc[owner[i]] = 1;
-                continue;
+        // each input's rotations (runs of equal owners) added in one pass
+        for (size_t i = 0; i < rot.size();) {
+            const int u = owner[i];
+            fides_ct* a = acc[u];
+            CtSumArgs sum{};
+            if (have_acc[u]) {
+                sum.in[0][0] = a->c0();
+                sum.in[1][0] = a->c1(N);
+                sum.n = 1;
+            } else if ((s = ct_reserve(c, a, level)) != FIDES_OK) {
+                return s;
             }
-            launch_elementwise(c->dev, EW_ADD, nl, 0, a->c0(), rot[i]->c0(), a->c0(), c->st);
-            launch_elementwise(c->dev, EW_ADD, nl, 0, a->c1(N), rot[i]->c1(N), a->c1(N), c->st);
+            for (; i < rot.size() && owner[i] == u && sum.n < kMaxSum; ++i, ++sum.n) {
+                sum.in[0][sum.n] = rot[i]->c0();
+                sum.in[1][sum.n] = rot[i]->c1(N);
+            }
+            sum.out[0] = a->c0();
+            sum.out[1] = a->c1(N);
+            have_acc[u] = 1;
+            launch_ct_sum(c->dev, nl, sum, c->st);
         }
     }
     for (int u = 0; u < nx; ++u) {

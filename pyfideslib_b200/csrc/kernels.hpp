@@ -177,12 +177,33 @@ void launch_ext_sum(const DevCtx& ctx, const ExtSumArgs& args, cudaStream_t st);
 enum { EW_ADD = 0, EW_SUB = 1, EW_NEG = 2, EW_MUL = 3, EW_COPY = 4 };
 void launch_elementwise(const DevCtx& ctx, int op, int n, int q0, const uint64_t* a, const uint64_t* b,
                         uint64_t* out, cudaStream_t st);
-// out = a * c_j (+ b) with one constant per limb from a device table [n][2] (value, Shoup)
-void launch_scalar_mac(const DevCtx& ctx, int n, const uint64_t* a, const uint64_t* cj, const uint64_t* b,
-                       uint64_t* out, cudaStream_t st);
-// out = a + c_j with one constant per limb (device table [n])
-void launch_scalar_add(const DevCtx& ctx, int n, const uint64_t* a, const uint64_t* cj, uint64_t* out,
-                       cudaStream_t st);
+// the same on both components of a ciphertext in one launch, an operation each
+// (o[1] null: component 0 alone)
+struct EwArgs {
+    const uint64_t* a[2];
+    const uint64_t* b[2];
+    uint64_t* o[2];
+    int op[2];
+};
+void launch_elementwise2(const DevCtx& ctx, int n, int q0, const EwArgs& args, cudaStream_t st);
+// One constant per limb (value, Shoup companion) on both components: times it,
+// or (mul false) component 0 plus it.
+constexpr int kMaxLinLimbs = 64;
+struct CtScalarArgs {
+    const uint64_t* a[2];
+    uint64_t* o[2];
+    int q0;  // prime of limb 0
+    uint64_t c[kMaxLinLimbs][2];
+};
+void launch_ct_scalar(const DevCtx& ctx, bool mul, int nlimbs, const CtScalarArgs& args, cudaStream_t st);
+// out = sum of n ciphertexts, both components (out may be one of them)
+constexpr int kMaxSum = kMaxBatch + 1;
+struct CtSumArgs {
+    const uint64_t* in[2][kMaxSum];
+    uint64_t* out[2];
+    int n;
+};
+void launch_ct_sum(const DevCtx& ctx, int nlimbs, const CtSumArgs& args, cudaStream_t st);
 // Plaintext dot product of ciphertexts (BSGS inner sums):
 //   o0 = sum_k c0[k] * p[k],  o1 = sum_k c1[k] * p[k]   (+ o0 / o1 when accumulate)
 // over limbs 0..nlimbs-1 with one 128-bit accumulator per output, n <= kMaxBatch.
@@ -201,7 +222,6 @@ void launch_dot_pt(const DevCtx& ctx, int nlimbs, const DotArgs& args, cudaStrea
 // added to component 0:
 //   out0 = sum_k z_k in0_k + add0_j,   out1 = sum_k z_k in1_k   over limbs 0..nlimbs-1.
 constexpr int kMaxLin = 8;
-constexpr int kMaxLinLimbs = 64;
 struct LinArgs {
     const uint64_t* in0[kMaxLin];
     const uint64_t* in1[kMaxLin];

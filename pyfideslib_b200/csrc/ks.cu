@@ -657,48 +657,58 @@ void launch_moddown_conv(const DevCtx& ctx, int level, int nb, const MdArgs& a, 
 // ---------------------------------------------------------------------------
 // element-wise
 // ---------------------------------------------------------------------------
-template <int OP>
-__global__ void k_elementwise(const __grid_constant__ DevCtx ctx, int q0, const uint64_t* __restrict__ a,
-                              const uint64_t* __restrict__ b, uint64_t* __restrict__ out) {
-    pdl_trigger();
-    pdl_wait();
-    const int limb = blockIdx.y;
-    const PrimeConst pc = ctx.pc[q0 + limb];
-    const size_t i = (size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2;
-    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(a + i);
-    ulonglong2 r;
-    if constexpr (OP == EW_COPY) {
-        r = x;
-    } else if constexpr (OP == EW_NEG) {
+__device__ __forceinline__ ulonglong2 ew_apply(int op, const ulonglong2 x, const uint64_t* b, size_t i,
+                                               const PrimeConst& pc) {
+    ulonglong2 r = x;
+    if (op == EW_COPY) return r;
+    if (op == EW_NEG) {
         r.x = neg_mod(x.x, pc.p);
         r.y = neg_mod(x.y, pc.p);
-    } else {
-        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(b + i);
-        if constexpr (OP == EW_ADD) {
-            r.x = add_mod(x.x, y.x, pc.p);
-            r.y = add_mod(x.y, y.y, pc.p);
-        } else if constexpr (OP == EW_SUB) {
-            r.x = sub_mod(x.x, y.x, pc.p);
-            r.y = sub_mod(x.y, y.y, pc.p);
-        } else {
-            r.x = mul_mod(x.x, y.x, pc);
-            r.y = mul_mod(x.y, y.y, pc);
-        }
+        return r;
     }
-    *reinterpret_cast<ulonglong2*>(out + i) = r;
+    const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(b + i);
+    if (op == EW_ADD) {
+        r.x = add_mod(x.x, y.x, pc.p);
+        r.y = add_mod(x.y, y.y, pc.p);
+    } else if (op == EW_SUB) {
+        r.x = sub_mod(x.x, y.x, pc.p);
+        r.y = sub_mod(x.y, y.y, pc.p);
+    } else if (pc.p < kFpPrimeBound) {
+        const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
+        r.x = fp_to_u(fp_mulmod(as_f64(fp_from_u(x.x)), as_f64(fp_from_u(y.x)), p, pinv), p, pinv);
+        r.y = fp_to_u(fp_mulmod(as_f64(fp_from_u(x.y)), as_f64(fp_from_u(y.y)), p, pinv), p, pinv);
+    } else {
+        r.x = mul_mod(x.x, y.x, pc);
+        r.y = mul_mod(x.y, y.y, pc);
+    }
+    return r;
+}
+
+// One operation per component (grid z): a ciphertext operation is one launch.
+__global__ void k_elementwise(const __grid_constant__ DevCtx ctx, int q0, const __grid_constant__ EwArgs args) {
+    pdl_trigger();
+    pdl_wait();
+    const int limb = blockIdx.y, h = blockIdx.z;
+    const PrimeConst pc = ctx.pc[q0 + limb];
+    const size_t i = (size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2;
+    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(args.a[h] + i);
+    *reinterpret_cast<ulonglong2*>(args.o[h] + i) = ew_apply(args.op[h], x, args.b[h], i, pc);
+}
+
+void launch_elementwise2(const DevCtx& ctx, int n, int q0, const EwArgs& args, cudaStream_t st) {
+    if (n <= 0) return;
+    count_launches(1);
+    launch_pdl(k_elementwise, dim3(ctx.N / 256, n, args.o[1] ? 2 : 1), 128, 0, st, ctx, q0, args);
 }
 
 void launch_elementwise(const DevCtx& ctx, int op, int n, int q0, const uint64_t* a, const uint64_t* b,
                         uint64_t* out, cudaStream_t st) {
-    if (n <= 0) return;
-    dim3 g(ctx.N / 256, n);
-    switch (op) {
-        case EW_ADD: count_launches(1); launch_pdl(k_elementwise<EW_ADD>, g, 128, 0, st, ctx, q0, a, b, out); break;
-        case EW_SUB: count_launches(1); launch_pdl(k_elementwise<EW_SUB>, g, 128, 0, st, ctx, q0, a, b, out); break;
-        case EW_NEG: count_launches(1); launch_pdl(k_elementwise<EW_NEG>, g, 128, 0, st, ctx, q0, a, b, out); break;
-        case EW_MUL: count_launches(1); launch_pdl(k_elementwise<EW_MUL>, g, 128, 0, st, ctx, q0, a, b, out); break;
-        default: count_launches(1); launch_pdl(k_elementwise<EW_COPY>, g, 128, 0, st, ctx, q0, a, b, out); break;
-    }
+    EwArgs e{};
+    e.a[0] = a;
+    e.b[0] = b;
+    e.o[0] = out;
+    e.op[0] = op;
+    launch_elementwise2(ctx, n, q0, e, st);
 }
 
 // Extended-basis sums of key-switch results: for output u, the elements
@@ -732,56 +742,59 @@ void launch_ext_sum(const DevCtx& ctx, const ExtSumArgs& a, cudaStream_t st) {
     launch_pdl(k_ext_sum, dim3((ctx.N + 511) / 512, a.n + ctx.K, a.nout), 256, 0, st, ctx, a);
 }
 
-__global__ void k_scalar_mac(const __grid_constant__ DevCtx ctx, const uint64_t* __restrict__ a,
-                             const uint64_t* __restrict__ cj, const uint64_t* __restrict__ b,
-                             uint64_t* __restrict__ out) {
+// One constant per limb applied to both components of a ciphertext (grid z =
+// component), the constants in the kernel parameters: nothing is uploaded and
+// nothing waits.  MUL: both times (c, Shoup companion); else c is added to
+// component 0 and component 1 is copied.
+template <bool MUL>
+__global__ void k_ct_scalar(const __grid_constant__ DevCtx ctx, const __grid_constant__ CtScalarArgs args) {
     pdl_trigger();
     pdl_wait();
-    const int limb = blockIdx.y;
-    const PrimeConst pc = ctx.pc[limb];
-    const ulonglong2 c = __ldg(reinterpret_cast<const ulonglong2*>(cj) + limb);
+    const int limb = blockIdx.y, h = blockIdx.z;
+    const uint64_t p = ctx.pc[args.q0 + limb].p;
     const size_t i = (size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2;
-    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(a + i);
-    ulonglong2 r;
-    r.x = mul_shoup(x.x, c.x, c.y, pc.p);
-    r.y = mul_shoup(x.y, c.x, c.y, pc.p);
-    if (b) {
-        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(b + i);
-        r.x = add_mod(r.x, y.x, pc.p);
-        r.y = add_mod(r.y, y.y, pc.p);
+    ulonglong2 x = *reinterpret_cast<const ulonglong2*>(args.a[h] + i);
+    if constexpr (MUL) {
+        x.x = mul_shoup(x.x, args.c[limb][0], args.c[limb][1], p);
+        x.y = mul_shoup(x.y, args.c[limb][0], args.c[limb][1], p);
+    } else if (h == 0) {
+        x.x = add_mod(x.x, args.c[limb][0], p);
+        x.y = add_mod(x.y, args.c[limb][0], p);
     }
-    *reinterpret_cast<ulonglong2*>(out + i) = r;
+    *reinterpret_cast<ulonglong2*>(args.o[h] + i) = x;
 }
 
-void launch_scalar_mac(const DevCtx& ctx, int n, const uint64_t* a, const uint64_t* cj, const uint64_t* b,
-                       uint64_t* out, cudaStream_t st) {
-    if (n <= 0) return;
-    dim3 g(ctx.N / 256, n);
+void launch_ct_scalar(const DevCtx& ctx, bool mul, int nlimbs, const CtScalarArgs& args, cudaStream_t st) {
+    if (nlimbs <= 0 || nlimbs > kMaxLinLimbs) return;
+    const dim3 g(ctx.N / 256, nlimbs, 2);
     count_launches(1);
-    launch_pdl(k_scalar_mac, g, 128, 0, st, ctx, a, cj, b, out);
+    if (mul)
+        launch_pdl(k_ct_scalar<true>, g, 128, 0, st, ctx, args);
+    else
+        launch_pdl(k_ct_scalar<false>, g, 128, 0, st, ctx, args);
 }
 
-__global__ void k_scalar_add(const __grid_constant__ DevCtx ctx, const uint64_t* __restrict__ a,
-                             const uint64_t* __restrict__ cj, uint64_t* __restrict__ out) {
+// Sum of n ciphertexts (both components, grid z).
+__global__ void k_ct_sum(const __grid_constant__ DevCtx ctx, const __grid_constant__ CtSumArgs args) {
     pdl_trigger();
     pdl_wait();
-    const int limb = blockIdx.y;
-    const PrimeConst pc = ctx.pc[limb];
-    const uint64_t c = __ldg(cj + limb);
+    const int limb = blockIdx.y, h = blockIdx.z;
+    const uint64_t p = ctx.pc[limb].p;
     const size_t i = (size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2;
-    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(a + i);
-    ulonglong2 r;
-    r.x = add_mod(x.x, c, pc.p);
-    r.y = add_mod(x.y, c, pc.p);
-    *reinterpret_cast<ulonglong2*>(out + i) = r;
+    ulonglong2 s = *reinterpret_cast<const ulonglong2*>(args.in[h][0] + i);
+#pragma unroll 4
+    for (int k = 1; k < args.n; ++k) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(args.in[h][k] + i);
+        s.x = add_mod(s.x, v.x, p);
+        s.y = add_mod(s.y, v.y, p);
+    }
+    *reinterpret_cast<ulonglong2*>(args.out[h] + i) = s;
 }
 
-void launch_scalar_add(const DevCtx& ctx, int n, const uint64_t* a, const uint64_t* cj, uint64_t* out,
-                       cudaStream_t st) {
-    if (n <= 0) return;
-    dim3 g(ctx.N / 256, n);
+void launch_ct_sum(const DevCtx& ctx, int nlimbs, const CtSumArgs& args, cudaStream_t st) {
+    if (nlimbs <= 0 || args.n < 1 || args.n > kMaxSum) return;
     count_launches(1);
-    launch_pdl(k_scalar_add, g, 128, 0, st, ctx, a, cj, out);
+    launch_pdl(k_ct_sum, dim3(ctx.N / 256, nlimbs, 2), 128, 0, st, ctx, args);
 }
 
 // Plaintext dot product: each thread owns two coefficients of both halves,
