@@ -1418,25 +1418,41 @@ fides_status fides::linear_transform_batch(fides_ctx* c, int nx, const fides_ct*
         const double sc = x->scale * pts[0]->scale;
         const int nd = x->noise_deg + pts[0]->noise_deg, sl = x->slots;
         acc[u] = tmp.make();
+        // the giant steps' inner sums, as many per launch as its tables hold
+        DotArgs d{};
+        int nbaby = 0;
+        auto flush = [&]() {
+            launch_dot_pt(c->dev, nl, d, c->st);
+            d = DotArgs{};
+            nbaby = 0;
+        };
         for (auto& kv : groups) {
             const int gs = kv.first;
             const std::vector<int>& ks = kv.second;
             fides_ct* dst = gs == 0 ? acc[u] : tmp.make();
             s = ct_reserve(c, dst, level);
             if (s != FIDES_OK) return s;
-            for (size_t k0 = 0; k0 < ks.size(); k0 += kMaxBatch) {
-                DotArgs d{};
-                d.n = (int)std::min(ks.size() - k0, (size_t)kMaxBatch);
-                d.accumulate = k0 > 0;
-                for (int j = 0; j < d.n; ++j) {
+            for (size_t k0 = 0; k0 < ks.size(); k0 += kMaxDotTerms) {
+                const int cnt = (int)std::min(ks.size() - k0, (size_t)kMaxDotTerms);
+                // a sum's second part adds to the first: a later launch
+                if (d.nout && (k0 > 0 || d.nout == kMaxDotOut || d.start[d.nout] + cnt > kMaxDotTerms)) flush();
+                const int base = d.start[d.nout];
+                for (int j = 0; j < cnt; ++j) {
                     const fides_ct* b = bct[baby[ks[k0 + j]]];
-                    d.c0[j] = b->c0();
-                    d.c1[j] = b->c1(N);
-                    d.p[j] = pts[ks[k0 + j]]->m;
+                    int i = 0;
+                    while (i < nbaby && d.c0[i] != b->c0()) ++i;
+                    if (i == nbaby) {
+                        d.c0[i] = b->c0();
+                        d.c1[i] = b->c1(N);
+                        ++nbaby;
+                    }
+                    d.baby[base + j] = (uint8_t)i;
+                    d.p[base + j] = pts[ks[k0 + j]]->m;
                 }
-                d.o0 = dst->c0();
-                d.o1 = dst->c1(N);
-                launch_dot_pt(c->dev, nl, d, c->st);
+                d.accumulate[d.nout] = k0 > 0;
+                d.o0[d.nout] = dst->c0();
+                d.o1[d.nout] = dst->c1(N);
+                d.start[++d.nout] = base + cnt;
             }
             dst->level = level;
             dst->scale = sc;
@@ -1450,6 +1466,7 @@ fides_status fides::linear_transform_batch(fides_ctx* c, int nx, const fides_ct*
                 owner.push_back(u);
             }
         }
+        flush();
     }
     if (!inner.empty() && (c->giant_moddown == 2 || (c->giant_moddown == 1 && boot))) {
         s = giant_rotate_sum(c, level, inner, gidx, owner, acc, have_acc, tmp);

@@ -204,17 +204,21 @@ struct CtSumArgs {
     int n;
 };
 void launch_ct_sum(const DevCtx& ctx, int nlimbs, const CtSumArgs& args, cudaStream_t st);
-// Plaintext dot product of ciphertexts (BSGS inner sums):
-//   o0 = sum_k c0[k] * p[k],  o1 = sum_k c1[k] * p[k]   (+ o0 / o1 when accumulate)
-// over limbs 0..nlimbs-1 with one 128-bit accumulator per output, n <= kMaxBatch.
+// Plaintext dot products of ciphertexts (BSGS inner sums), several outputs per
+// launch:
+//   o0[u] = sum_k c0[baby[k]] * p[k],  o1[u] = sum_k c1[baby[k]] * p[k]
+// over the terms start[u] <= k < start[u + 1] (plus o0 / o1 where accumulate).
+constexpr int kMaxDotTerms = 64, kMaxDotOut = 16;
 struct DotArgs {
-    const uint64_t* c0[kMaxBatch];
-    const uint64_t* c1[kMaxBatch];
-    const uint64_t* p[kMaxBatch];
-    int n;
-    int accumulate;
-    uint64_t* o0;
-    uint64_t* o1;
+    const uint64_t* c0[kMaxDotTerms];  // distinct baby steps
+    const uint64_t* c1[kMaxDotTerms];
+    const uint64_t* p[kMaxDotTerms];
+    uint8_t baby[kMaxDotTerms];
+    uint8_t accumulate[kMaxDotOut];
+    int start[kMaxDotOut + 1];
+    int nout;
+    uint64_t* o0[kMaxDotOut];
+    uint64_t* o1[kMaxDotOut];
 };
 void launch_dot_pt(const DevCtx& ctx, int nlimbs, const DotArgs& args, cudaStream_t st);
 // Integer linear combination over ciphertext components, with per-limb

@@ -797,58 +797,94 @@ void launch_ct_sum(const DevCtx& ctx, int nlimbs, const CtSumArgs& args, cudaStr
     launch_pdl(k_ct_sum, dim3(ctx.N / 256, nlimbs, 2), 128, 0, st, ctx, args);
 }
 
-// Plaintext dot product: each thread owns two coefficients of both halves,
-// reads each plaintext term once for c0 and c1.  Products of residues below
-// 2^62 are below 2^124, so 15 of them plus a folded residue fit in 128 bits;
-// the accumulators are folded back to one residue every 15 terms.
+// Plaintext dot products (the inner sums of a baby-step giant-step transform,
+// one output per giant step): each thread owns two coefficients of both halves
+// and reads each plaintext term once for c0 and c1.  The outputs vary fastest
+// over the grid, then the tiles of a limb, then the limbs: the giant steps read
+// the same baby-step tiles at the same time, so a baby step comes from HBM once
+// per transform.  (One launch per giant step read every baby step from HBM
+// again: 8 launches of 46 us for 64 diagonals of 20 limbs at N = 2^16, 8 baby
+// steps of 21 MB each, 5.5 TB/s.)
+// Sums: exact FP64 products for primes below 2^50 (|r| <= 0.875p, centred every
+// seven terms, below 7.2p), else 128-bit ones folded every 15 terms (products of
+// residues below 2^62 are below 2^124).
 // Role in the reference: dotProductPt_ (CKKS/ElemenwiseBatchKernels.cu:651).
-__global__ void k_dot_pt(const __grid_constant__ DevCtx ctx, const __grid_constant__ DotArgs args) {
+__global__ void __launch_bounds__(128) k_dot_pt(const __grid_constant__ DevCtx ctx, const __grid_constant__ DotArgs args) {
     pdl_trigger();
     pdl_wait();
-    const int limb = blockIdx.y;
+    const int u = blockIdx.x, limb = blockIdx.z;
     const PrimeConst pc = ctx.pc[limb];
-    const size_t i = (size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2;
-    Acc128 a0, a1, b0, b1;
-    if (args.accumulate) {
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(args.o0 + i);
-        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(args.o1 + i);
-        a0.lo = x.x;
-        a1.lo = x.y;
-        b0.lo = y.x;
-        b1.lo = y.y;
+    const size_t i = (size_t)limb * ctx.N + (size_t)(blockIdx.y * blockDim.x + threadIdx.x) * 2;
+    const int k0 = args.start[u], k1 = args.start[u + 1];
+    ulonglong2 r0 = make_ulonglong2(0, 0), r1 = r0;
+    if (args.accumulate[u]) {
+        r0 = *reinterpret_cast<const ulonglong2*>(args.o0[u] + i);
+        r1 = *reinterpret_cast<const ulonglong2*>(args.o1[u] + i);
     }
-    int since = 0;
-#pragma unroll 1
-    for (int k = 0; k < args.n; ++k) {
-        const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(args.p[k] + i));
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(args.c0[k] + i);
-        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(args.c1[k] + i);
-        a0.mac(x.x, w.x);
-        a1.mac(x.y, w.y);
-        b0.mac(y.x, w.x);
-        b1.mac(y.y, w.y);
-        if (++since == 15) {
-            a0.lo = a0.reduce(pc), a0.hi = 0;
-            a1.lo = a1.reduce(pc), a1.hi = 0;
-            b0.lo = b0.reduce(pc), b0.hi = 0;
-            b1.lo = b1.reduce(pc), b1.hi = 0;
-            since = 0;
+    auto term = [&](int k, ulonglong2& w, ulonglong2& x, ulonglong2& y) {
+        const int b = args.baby[k];
+        w = __ldg(reinterpret_cast<const ulonglong2*>(args.p[k] + i));
+        x = *reinterpret_cast<const ulonglong2*>(args.c0[b] + i);
+        y = *reinterpret_cast<const ulonglong2*>(args.c1[b] + i);
+    };
+    if (pc.p < kFpPrimeBound) {
+        const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
+        auto conv = [](uint64_t v) { return as_f64(fp_from_u(v)); };
+        double a0 = conv(r0.x), a1 = conv(r0.y), b0 = conv(r1.x), b1 = conv(r1.y);
+        int since = 0;
+#pragma unroll 4
+        for (int k = k0; k < k1; ++k) {
+            ulonglong2 w, x, y;
+            term(k, w, x, y);
+            const double w0 = conv(w.x), w1 = conv(w.y);
+            a0 = __dadd_rn(a0, fp_mulmod(conv(x.x), w0, p, pinv));
+            a1 = __dadd_rn(a1, fp_mulmod(conv(x.y), w1, p, pinv));
+            b0 = __dadd_rn(b0, fp_mulmod(conv(y.x), w0, p, pinv));
+            b1 = __dadd_rn(b1, fp_mulmod(conv(y.y), w1, p, pinv));
+            if (++since == 7) {
+                a0 = fp_center(a0, p, pinv);
+                a1 = fp_center(a1, p, pinv);
+                b0 = fp_center(b0, p, pinv);
+                b1 = fp_center(b1, p, pinv);
+                since = 0;
+            }
         }
+        r0 = make_ulonglong2(fp_sum_to_u(a0, p, pinv), fp_sum_to_u(a1, p, pinv));
+        r1 = make_ulonglong2(fp_sum_to_u(b0, p, pinv), fp_sum_to_u(b1, p, pinv));
+    } else {
+        Acc128 a0, a1, b0, b1;
+        a0.lo = r0.x;
+        a1.lo = r0.y;
+        b0.lo = r1.x;
+        b1.lo = r1.y;
+        int since = 0;
+#pragma unroll 2
+        for (int k = k0; k < k1; ++k) {
+            ulonglong2 w, x, y;
+            term(k, w, x, y);
+            a0.mac(x.x, w.x);
+            a1.mac(x.y, w.y);
+            b0.mac(y.x, w.x);
+            b1.mac(y.y, w.y);
+            if (++since == 15) {
+                a0.lo = a0.reduce(pc), a0.hi = 0;
+                a1.lo = a1.reduce(pc), a1.hi = 0;
+                b0.lo = b0.reduce(pc), b0.hi = 0;
+                b1.lo = b1.reduce(pc), b1.hi = 0;
+                since = 0;
+            }
+        }
+        r0 = make_ulonglong2(a0.reduce(pc), a1.reduce(pc));
+        r1 = make_ulonglong2(b0.reduce(pc), b1.reduce(pc));
     }
-    ulonglong2 r;
-    r.x = a0.reduce(pc);
-    r.y = a1.reduce(pc);
-    *reinterpret_cast<ulonglong2*>(args.o0 + i) = r;
-    r.x = b0.reduce(pc);
-    r.y = b1.reduce(pc);
-    *reinterpret_cast<ulonglong2*>(args.o1 + i) = r;
+    *reinterpret_cast<ulonglong2*>(args.o0[u] + i) = r0;
+    *reinterpret_cast<ulonglong2*>(args.o1[u] + i) = r1;
 }
 
 void launch_dot_pt(const DevCtx& ctx, int nlimbs, const DotArgs& args, cudaStream_t st) {
-    if (nlimbs <= 0 || args.n <= 0 || args.n > kMaxBatch) return;
-    dim3 g(ctx.N / 256, nlimbs);
+    if (nlimbs <= 0 || args.nout <= 0) return;
     count_launches(1);
-    launch_pdl(k_dot_pt, g, 128, 0, st, ctx, args);
+    launch_pdl(k_dot_pt, dim3(args.nout, ctx.N / 256, nlimbs), 128, 0, st, ctx, args);
 }
 
 // Integer linear combination (leaf sums of polynomial evaluation, integer
