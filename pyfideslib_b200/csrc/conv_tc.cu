@@ -122,8 +122,9 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 struct __align__(16) TcMod {
     uint64_t np;   // -p
     uint32_t M;
-    uint32_t shk;  // s - 16, and k << 16
+    uint32_t shk;  // s - 16 in bits 0-4, kTcNear, k << 16
 };
+constexpr uint32_t kTcNear = 0x100;  // fused ModDown: q_level < 2p
 __device__ __forceinline__ TcMod tc_mod(const PrimeConst& pc, int cnt) {
     const int bits = 64 - __clzll((long long)pc.p);
     const int s = max(16, bits + (32 - __clz(2040 * cnt)) - 32);
@@ -261,7 +262,7 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
     k_conv_tc(const __grid_constant__ DevCtx ctx, int level, const __grid_constant__ TcArgs args) {
     extern __shared__ __align__(1024) uint8_t smem[];
     pdl_trigger();
-    const int ntiles = ctx.N / kTcRows;
+    const int tlog = ctx.logN - 7, ntiles = 1 << tlog;  // tiles of kTcRows = 2^7 coefficients
     // ModDown with the top limb (target 0 = prime `level`); both halves alike
     const bool fused = MD && args.md.ttop[0] != nullptr;
     const int d = MD ? 0 : blockIdx.y;
@@ -275,16 +276,16 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
     // element offset (words) and half of item `it`
     auto item_off = [&](int it, int& half) -> size_t {
         if (MD) {
-            const int bh = it / ntiles;
+            const int bh = it >> tlog;
             half = bh & 1;
             return (size_t)(bh >> 1) * args.md.bstride;
         }
         half = 0;
-        return (size_t)(it / ntiles) * args.bstride;
+        return (size_t)(it >> tlog) * args.bstride;
     };
     auto item_in = [&](int it) -> const uint64_t* {
         int h;
-        const size_t off = item_off(it, h) + (size_t)(it % ntiles) * kTcRows;
+        const size_t off = item_off(it, h) + (size_t)(it & (ntiles - 1)) * kTcRows;
         return MD ? args.md.y[h] + off : args.xt + off + (size_t)lo * ctx.N;
     };
     const uint32_t lbo_b = sh.lbo_b();
@@ -302,7 +303,11 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
         const PrimeConst pc = ctx.pc[sh.tprime(ctx, min(m, ntar - 1))];
         sP[m] = pc;
         sMod[m] = tc_mod(pc, cnt);
-        if (MD) sOm[m] = pc.p - csub(reduce64_lazy(ctx.pc[level].p, pc), pc.p);
+        if (MD) {
+            const uint64_t ql = ctx.pc[level].p;
+            sOm[m] = pc.p - csub(reduce64_lazy(ql, pc), pc.p);
+            if (ql < 2 * pc.p) sMod[m].shk |= kTcNear;
+        }
     }
     // A: zero once (limbs cnt..4*CK-1 stay zero)
     for (int i = threadIdx.x; i < 2 * CK * (int)kTcLboA / 16; i += kTcThreads)
@@ -358,23 +363,13 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
     for (int it = it_begin; it < it_end && ok; ++it) {
         int half;
         const size_t boff = item_off(it, half);
-        const size_t j = (size_t)(it % ntiles) * kTcRows + row;  // this thread's coefficient
+        const size_t j = (size_t)(it & (ntiles - 1)) * kTcRows + row;  // this thread's coefficient
         // this row's outputs: target m at obase + m N (the fused ModDown's target 0
         // is the top limb, which has none)
         uint64_t* obase = MD ? args.md.w[half] + boff + j - (fused ? ctx.N : 0)
                              : args.dig + boff + (size_t)d * args.dig_stride * ctx.N + j;
         uint64_t tl = 0, ql = 0;
         bool up = false;  // tl stands for tl - q_l
-        auto finish = [&](int m, uint64_t v) {
-            if (MD && fused) {
-                // v = P^-1 conv_q (folded into the constants); SwitchModulus(tl, q_l -> q)
-                const PrimeConst pc = sP[m];
-                uint64_t sw = up ? tl + sOm[m] : tl;
-                if (pc.p < ql) sw = csub(reduce64_lazy(sw, pc), pc.p);
-                v = add_mod(v, sw, pc.p);
-            }
-            obase[(size_t)((uint32_t)m * (uint32_t)ctx.N)] = v;
-        };
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
             const int e = threadIdx.x + q * kTcThreads;
@@ -430,22 +425,52 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
             // second group.  The four reductions are independent and run before
             // any store, so that their latencies overlap: with branches between
             // them the epilogue waited two issue slots per instruction at 16
-            // warps per SM.
+            // warps per SM.  (24 or 32 warps per SM with two targets each were 1-2%
+            // slower over a whole HMult.)
 #pragma unroll 1
             for (int g = 4 * wh; g < nt; g += 8) {
                 uint32_t c[32];
                 tmem_ld32(t_lane + (uint32_t)(g * kTcCols), c);
                 const int m = m0 + g;
                 TcMod md[4];
+                uint32_t near = kTcNear;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) md[u] = sMod[min(m + u, ntar2 - 1)];
+                for (int u = 0; u < 4; ++u) {
+                    md[u] = sMod[min(m + u, ntar2 - 1)];
+                    near &= md[u].shk;
+                }
                 tmem_wait_ld();
                 uint64_t v[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) v[u] = reduce_cols(c + 8 * u, md[u]);
+                if (MD && fused) {
+                    // v = P^-1 conv_q (folded into the constants) + SwitchModulus(tl, q_l -> q)
+                    if (near) {
+                        // q_l < 2q, as in any chain of like-sized primes: the centred
+                        // tl lies in (-q, q) and one conditional addition does (with a
+                        // Barrett step per target of q < q_l one HMult of N = 2^16,
+                        // L = 30 took 261 us against 259, 32 of them 6172 against 6112)
+                        const uint64_t ctl = up ? tl - ql : tl;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const uint64_t s = v[u] + ctl + (up ? 0 : md[u].np);  // v + tl' - q or v + tl': [-q, q)
+                            v[u] = (int64_t)s < 0 ? s - md[u].np : s;
+                        }
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const PrimeConst pc = sP[min(m + u, ntar2 - 1)];
+                            uint64_t sw = up ? tl + sOm[min(m + u, ntar2 - 1)] : tl;
+                            if (pc.p < ql) sw = csub(reduce64_lazy(sw, pc), pc.p);
+                            v[u] = add_mod(v[u], sw, pc.p);
+                        }
+                    }
+                }
+                const int lim = min(nt - g, ntar - m);
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
-                    if (g + u < nt && m + u < ntar && !(MD && fused && m + u == 0)) finish(m + u, v[u]);
+                    if (u < lim && !(MD && fused && u == 0 && m == 0))
+                        obase[(size_t)((uint32_t)(m + u) * (uint32_t)ctx.N)] = v[u];
             }
         }
     }
