@@ -114,11 +114,11 @@ fides_status fides_set_conv_accumulator(fides_ctx* ctx, int accumulator);
  * measurements and tests).  Bit 0: the digit products of primes below 2^50
  * are summed exactly on the FP64 pipes (else 128-bit integer sums).  Bit 1:
  * HMult's inner product runs in the epilogue of the ModUp digits' NTT row
- * pass (else in its own kernel).  Bit 2: the same for HMult batches of eight
- * or more elements only.  Bit 3: that fused row pass in two launches, the
- * ciphertext-prime outputs (one digit tile less in shared memory) at 3 CTAs
- * per SM and the special-prime outputs at 2 (forward NTT variant 9 only).
- * Default 13 (FP64 sums, fused for batches of 8+, split launch). */
+ * pass (else in its own kernel).  Bit 2: the same for large HMult batches
+ * only (768 MiB of digits and more).  Bit 3: that fused row pass in two
+ * launches, the special-prime outputs and the ciphertext-prime outputs (one
+ * digit tile less in shared memory, more CTAs per SM).
+ * Default 13 (FP64 sums, fused for large batches, split launch). */
 fides_status fides_set_keyswitch_variant(fides_ctx* ctx, int variant);
 /* Giant steps of the baby-step giant-step linear transforms: each input's
  * giant-step rotations are added in the extended basis (Q and the special

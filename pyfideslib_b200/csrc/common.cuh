@@ -52,9 +52,9 @@ struct DevCtx {
     int ks_variant;              // key-switch inner product: bit 0 set: FP64 sums on primes below 2^50
                                  // (else integer sums); bit 1 set: HMult's inner product runs in the
                                  // epilogue of the ModUp digits' NTT row pass (else its own kernel);
-                                 // bit 2 set: the same for HMult batches of 8 or more elements;
-                                 // bit 3 set: that fused row pass in two launches (ciphertext-
-                                 // prime outputs at 3 CTAs per SM, special-prime outputs at 2)
+                                 // bit 2 set: the same for large HMult batches only (engine.cpp);
+                                 // bit 3 set: that fused row pass in two launches (special-prime
+                                 // outputs, then ciphertext-prime outputs)
     int conv_variant;            // base conversions: 0 2 coefficients/thread 128-bit sums, 1 the same with
                                  // split 32-bit products (moduli < 2^60), 2 one coefficient/thread,
                                  // 3 and 4 ModUp and ModDown on the tensor cores (int8 split, 32
@@ -98,7 +98,6 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 struct LimbSeg {
     const uint64_t* in;
     const uint64_t* in2;
-    const uint64_t* in3;
     uint64_t* out;
     int count;
     int skip_lo, skip_cnt;
@@ -108,8 +107,8 @@ struct LimbSeg {
     int8_t lmode;  // transform prologue mode (FL_* forward, IL_* inverse)
     int8_t smode;  // transform epilogue mode (FS_* forward, IS_* inverse)
     int8_t out_tab;  // t > 0: batch element b writes to LimbMap::bout[t - 1][b] (+ limb offset)
-    int8_t pad;
-    size_t bstride;  // batch element b adds b * bstride words to in/in2/in3/out
+    int8_t in_tab;   // 1: batch element b reads in and in2 from LimbMap::bin[0][b] and bin[1][b] (+ limb offset)
+    size_t bstride;  // batch element b adds b * bstride words to in/in2/out
 };
 
 struct LimbMap {
@@ -118,12 +117,12 @@ struct LimbMap {
     int nb;  // batch elements (gridDim.z); 0 means 1
     LimbSeg seg[kMaxSeg];
     uint64_t* bout[2][kMaxBatch];
+    const uint64_t* bin[2][kMaxBatch];
 };
 
 struct LimbRef {
     const uint64_t* in;
     const uint64_t* in2;
-    const uint64_t* in3;
     uint64_t* out;
     int prime;
     int level;
@@ -143,7 +142,10 @@ __device__ __forceinline__ LimbRef resolve_limb(const LimbMap& m, int f, int b, 
     const size_t bo = (size_t)b * g.bstride;
     r.in = g.in ? g.in + bo + (g.in_stride_zero ? 0 : off) : nullptr;
     r.in2 = g.in2 ? g.in2 + bo + off : nullptr;
-    r.in3 = g.in3 ? g.in3 + bo + off : nullptr;
+    if (g.in_tab > 0) {
+        r.in = m.bin[0][b] + off;
+        r.in2 = m.bin[1][b] + off;
+    }
     if (g.out_tab > 0)
         r.out = m.bout[g.out_tab - 1][b] + off;
     else

@@ -206,15 +206,13 @@ fides_status consume_device_error(fides_ctx* c, cudaStream_t st) {
     return FIDES_OK;
 }
 
-LimbMap map_single(const uint64_t* in, uint64_t* out, int count, int nq, int q0, int level, const uint64_t* in2,
-                   const uint64_t* in3) {
+LimbMap map_single(const uint64_t* in, uint64_t* out, int count, int nq, int q0, int level, const uint64_t* in2) {
     LimbMap m{};
     m.nseg = 1;
     m.total = count;
     LimbSeg& s = m.seg[0];
     s.in = in;
     s.in2 = in2;
-    s.in3 = in3;
     s.out = out;
     s.count = count;
     s.skip_lo = count;
@@ -509,7 +507,7 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
     d.dnum = c->dnum;
     d.alpha = c->alpha;
     d.ntt_variant = d.intt_variant = d.conv_variant = 0;  // chosen by the autotuner
-    d.ks_variant = 1 | 4 | 8;  // FP64 sums; fused into the row pass (split launch) for batches of 8 or more
+    d.ks_variant = 1 | 4 | 8;  // FP64 sums; fused into the row pass (split launch) for large batches
     d.pc = (const PrimeConst*)(base + parts[i_pc].off);
     d.fwd_tw = (const uint64_t*)(base + parts[i_fwd].off);
     d.inv_tw = (const uint64_t*)(base + parts[i_inv].off);
@@ -582,7 +580,7 @@ fides_status ws_reserve(fides_ctx* c, Workspace& w, int cap) {
     w.st = keep;
     const size_t L = c->L, K = c->K, N = c->N;
     w.dig_stride = L + K;
-    const size_t limbs = 4 * L /*E0,E1,E2,XT*/ + c->dnum * w.dig_stride /*DIG*/ + 2 * (L + K) /*XB,XA*/ +
+    const size_t limbs = L /*XT*/ + c->dnum * w.dig_stride /*DIG*/ + 2 * (L + K) /*XB,XA*/ +
                          2 * L /*W*/ + 2 /*T*/;
     w.stride = limbs * N;
     if (cudaMalloc((void**)&w.base, w.stride * 8 * (size_t)cap) != cudaSuccess) {
@@ -597,9 +595,6 @@ fides_status ws_reserve(fides_ctx* c, Workspace& w, int cap) {
         p += n * N;
         return r;
     };
-    w.E0 = take(L);
-    w.E1 = take(L);
-    w.E2 = take(L);
     w.XT = take(L);
     w.DIG = take(c->dnum * w.dig_stride);
     w.XB = take(L + K);

@@ -65,8 +65,7 @@ struct Workspace {
     size_t stride = 0;  // words per element
     int cap = 0;
     size_t dig_stride = 0;  // limbs per digit in DIG
-    uint64_t *E0 = nullptr, *E1 = nullptr, *E2 = nullptr, *XT = nullptr, *DIG = nullptr, *XB = nullptr,
-             *XA = nullptr, *W = nullptr, *T = nullptr;
+    uint64_t *XT = nullptr, *DIG = nullptr, *XB = nullptr, *XA = nullptr, *W = nullptr, *T = nullptr;
 };
 
 // Moduli and host copies of the per-prime constants.
@@ -167,7 +166,7 @@ fides_status build_context(fides_ctx* c, const fides_params* p);
 bool select_moduli(const fides_params* prm, std::vector<uint64_t>& q, std::vector<uint64_t>& p);
 void free_context(fides_ctx* c);
 LimbMap map_single(const uint64_t* in, uint64_t* out, int count, int nq, int q0, int level = -1,
-                   const uint64_t* in2 = nullptr, const uint64_t* in3 = nullptr);
+                   const uint64_t* in2 = nullptr);
 fides_status ws_reserve(fides_ctx* c, Workspace& w, int cap);
 // (Re)allocate a switching key's storage: b only when seeded, b and a otherwise.
 fides_status key_alloc(fides_ctx* c, SwitchKey& k, bool seeded);

@@ -7,7 +7,8 @@
 // :458-571 fusedHoistRotate; Ciphertext.cpp:409-622, :756-926, :1053-1226):
 //   tensor -> INTT -> ModUp conversion -> NTT -> inner product with the key
 //   -> INTT of the special limbs -> ModDown conversion -> NTT -> combine
-//   (-> rescale).  Here ModDown and Rescale share their NTT (see
+//   (-> rescale).  Here the tensor product is formed inside the first INTT's load
+//   and the inner product, ModDown and Rescale share their NTT (see
 //   moddown_finish) and every step runs once for the whole batch.
 #include "context.hpp"
 
@@ -15,11 +16,15 @@ namespace fides {
 
 namespace {
 
-// batch size from which the key switch fused into the digits' row pass wins
-// (B200, N=2^16, L=30, dnum=3, ms per batched step unfused / fused: 4 pairs
-// 0.986 / 0.997, 8 pairs 1.854 / 1.844, 16 pairs 3.578 / 3.529, 32 pairs
-// 7.008 / 6.886)
-constexpr int kFuseMinBatch = 8;
+// Digit words of a batch from which HMult's inner product runs fused into the
+// digits' row pass: 768 MiB, about six times the L2.  The fused kernel's few long
+// warps per SM are slower in themselves; what it saves is the digits' return
+// trip to HBM, and under the power cap that trip costs clock too.  Back to back
+// for a second each, us unfused / fused, N = 2^16: L = 30 (87 digit limbs) 8 pairs
+// 1586 / 1649, 16 pairs 3110 / 3102, 24 pairs 4626 / 4607, 32 pairs 6161 / 6094;
+// L = 20 (61) 12 pairs 1659 / 1713, 24 pairs 3261 / 3223, 32 pairs 4298 / 4283;
+// N = 2^15, L = 16 (50) 32 pairs 1758 / 1786.
+constexpr size_t kFuseMinWords = (size_t)96 << 20;
 
 LimbSeg seg_ws(const uint64_t* in, uint64_t* out, int count, int nq, int q0, int level, size_t bstride) {
     LimbSeg g{};
@@ -35,7 +40,7 @@ LimbSeg seg_ws(const uint64_t* in, uint64_t* out, int count, int nq, int q0, int
 }
 
 // Special limbs of XB / XA -> INTT scaled by (P/p_k)^-1 (in place), and, for
-// the fused rescale, INTT(e_l + P^-1 x_l) of both halves into T.
+// the fused rescale, the INTT of both halves' top limbs into T.
 void special_intt(fides_ctx* c, Workspace& w, int level, int nb, bool with_top) {
     const int n = level + 1, N = c->N;
     LimbMap m{};
@@ -49,11 +54,9 @@ void special_intt(fides_ctx* c, Workspace& w, int level, int nb, bool with_top) 
         m.total += c->K;
     }
     if (with_top) {
-        const uint64_t* es[2] = {w.E0, w.E1};
         for (int s = 0; s < 2; ++s) {
-            LimbSeg g = seg_ws(es[s] + (size_t)level * N, w.T + (size_t)s * N, 1, 1, level, level, w.stride);
-            g.in2 = xs[s] + (size_t)level * N;
-            g.lmode = IL_AXPY_PINV;
+            LimbSeg g = seg_ws(xs[s] + (size_t)level * N, w.T + (size_t)s * N, 1, 1, level, level, w.stride);
+            g.lmode = IL_PLAIN;
             g.smode = IS_PLAIN;
             m.seg[m.nseg++] = g;
             m.total += 1;
@@ -62,11 +65,12 @@ void special_intt(fides_ctx* c, Workspace& w, int level, int nb, bool with_top) 
     ntt_inverse(c->dev, m, -1, -1, w.st);
 }
 
-// ModDown of XB -> out0, XA -> out1 for every element, adding e0/e1 (E0/E1 of
-// the workspace) when `add_e`; with `rescale` the result is also rescaled:
-//   out = Rescale(e + ModDown(x)), computed as one NTT per output limb.
+// ModDown of XB -> out0, XA -> out1 for every element.  product: the ciphertext
+// limbs hold e + P^-1 x already (launch_ks_hmult); with `rescale` (products
+// only) the result is also rescaled: out = Rescale(e + ModDown(x)), computed as
+// one NTT per output limb.
 void moddown_finish(fides_ctx* c, Workspace& w, int level, int nb, uint64_t* const* out0, uint64_t* const* out1,
-                    bool add_e, bool rescale) {
+                    bool product, bool rescale) {
     const int n = level + 1, N = c->N, L = c->L;
     special_intt(c, w, level, nb, rescale);
     MdArgs md{};
@@ -82,12 +86,10 @@ void moddown_finish(fides_ctx* c, Workspace& w, int level, int nb, uint64_t* con
     m.nb = nb;
     m.nseg = 2;
     const uint64_t* xs[2] = {w.XB, w.XA};
-    const uint64_t* es[2] = {w.E0, w.E1};
     const int nout = rescale ? level : n;
     for (int s = 0; s < 2; ++s) {
         LimbSeg g = seg_ws(w.W + (size_t)s * L * N, nullptr, nout, nout, 0, level, w.stride);
         g.in2 = xs[s];
-        g.in3 = add_e ? es[s] : nullptr;
         g.out_tab = (int8_t)(s + 1);
         m.seg[s] = g;
         m.total += nout;
@@ -96,7 +98,7 @@ void moddown_finish(fides_ctx* c, Workspace& w, int level, int nb, uint64_t* con
         m.bout[0][b] = out0[b];
         m.bout[1][b] = out1[b];
     }
-    ntt_forward(c->dev, m, FL_PLAIN, rescale ? FS_MDRS : FS_MODDOWN, w.st);
+    ntt_forward(c->dev, m, FL_PLAIN, rescale ? FS_RESCALE : product ? FS_SUBP : FS_MODDOWN, w.st);
 }
 
 }  // namespace
@@ -147,65 +149,47 @@ void eng_hmult(fides_ctx* c, Workspace& w, int level, int nb, const uint64_t* co
                const uint64_t* const* b0, const uint64_t* const* b1, uint64_t* const* out0, uint64_t* const* out1,
                bool rescale, const SwitchKey& key) {
     const int n = level + 1;
-    TensorArgs ta{};
-    for (int b = 0; b < nb; ++b) {
-        ta.a0[b] = a0[b];
-        ta.a1[b] = a1[b];
-        ta.b0[b] = b0[b];
-        ta.b1[b] = b1[b];
-    }
-    ta.e0 = w.E0;
-    ta.e1 = w.E1;
-    ta.e2 = w.E2;
-    ta.bstride = w.stride;
-    launch_tensor(c->dev, n, nb, ta, w.st);
-    // scaled INTT of E2 (workspace: batch dimension with the element stride)
+    // fused inner product: forced (bit 1), or for batches of at least
+    // kFuseMinWords words of digits (bit 2)
+    const int nd = level / c->alpha + 1;
+    const size_t words = (size_t)nb * (size_t)(nd * (n + c->K) - n) * (size_t)c->N;
+    const bool fuse = ((c->dev.ks_variant & 2) || ((c->dev.ks_variant & 4) && words >= kFuseMinWords)) &&
+                      ntt_rows_keyswitch_supported(c->dev) && key.a != nullptr;
+    // scaled INTT of a1 b1 (the product in its load) and ModUp conversion
     LimbMap im{};
     im.nb = nb;
-    im.seg[im.nseg++] = seg_ws(w.E2, w.XT, n, n, 0, level, w.stride);
+    LimbSeg g = seg_ws(nullptr, w.XT, n, n, 0, level, w.stride);
+    g.in_tab = 1;
+    im.seg[im.nseg++] = g;
     im.total = n;
-    ntt_inverse(c->dev, im, IL_PLAIN, IS_MODUP, w.st);
-    // fused inner product: forced (bit 1), or for batches of at least
-    // kFuseMinBatch elements (bit 2; a small batch's fused launch is a few
-    // waves of long CTAs at 2 per SM and measured slower than the two kernels)
-    const bool fuse = ((c->dev.ks_variant & 2) || ((c->dev.ks_variant & 4) && nb >= kFuseMinBatch)) &&
-                      ntt_rows_keyswitch_supported(c->dev) && key.a != nullptr;
-    if (fuse) {
-        // ModUp conversion and the digits' column pass; the row pass runs
-        // fused with the inner product, so the digits' evaluation limbs never
-        // reach HBM
-        launch_modup_conv(c->dev, level, nb, w.XT, w.DIG, w.dig_stride, w.stride, w.st);
-        ntt_forward_cols(c->dev, digit_map(c, w, level, nb), FL_PLAIN, w.st);
-        KsFuseArgs fa{};
-        fa.dig = w.DIG;
-        fa.own = w.E2;
-        fa.kb = key.b;
-        fa.ka = key.a;
-        fa.xb = w.XB;
-        fa.xa = w.XA;
-        fa.dig_stride = w.dig_stride;
-        fa.bstride = w.stride;
-        fa.level = level;
-        fa.fp_sums = c->dev.ks_variant & 1;
-        ntt_rows_keyswitch(c->dev, fa, nb, w.st);
-        moddown_finish(c, w, level, nb, out0, out1, true, rescale && level > 0);
-        return;
-    }
-    modup_from_xt(c, w, level, nb);
-    KsArgs ka{};
+    KsHmultArgs ka{};
     for (int b = 0; b < nb; ++b) {
-        ka.own[b] = w.E2 + (size_t)b * w.stride;
-        ka.kb[b] = key.b;
-        ka.ka[b] = key.a;
-        ka.a_seed[b] = key.a ? 0 : uniform_stream(key.a_seed, 0);
+        im.bin[0][b] = ka.a1[b] = a1[b];
+        im.bin[1][b] = ka.b1[b] = b1[b];
+        ka.a0[b] = a0[b];
+        ka.b0[b] = b0[b];
     }
     ka.dig = w.DIG;
+    ka.kb = key.b;
+    ka.ka = key.a;
+    ka.a_seed = key.a ? 0 : uniform_stream(key.a_seed, 0);
     ka.xb = w.XB;
     ka.xa = w.XA;
     ka.dig_stride = w.dig_stride;
     ka.bstride = w.stride;
-    ka.dig_bstride = w.stride;
-    launch_ks_inner(c->dev, level, nb, ka, true, w.st);
+    ka.level = level;
+    ka.fp_sums = c->dev.ks_variant & 1;
+    ntt_inverse(c->dev, im, IL_MUL, IS_MODUP, w.st);
+    launch_modup_conv(c->dev, level, nb, w.XT, w.DIG, w.dig_stride, w.stride, w.st);
+    // the digits' NTT and the inner product with the rest of the tensor product;
+    // fused, the digits' evaluation limbs do not reach HBM
+    if (fuse) {
+        ntt_forward_cols(c->dev, digit_map(c, w, level, nb), FL_PLAIN, w.st);
+        ntt_rows_keyswitch(c->dev, ka, nb, w.st);
+    } else {
+        ntt_forward(c->dev, digit_map(c, w, level, nb), FL_PLAIN, FS_PLAIN, w.st);
+        launch_ks_hmult(c->dev, nb, ka, w.st);
+    }
     moddown_finish(c, w, level, nb, out0, out1, true, rescale && level > 0);
 }
 
@@ -232,7 +216,7 @@ void eng_rotate(fides_ctx* c, Workspace& w, int level, int nb, const uint64_t* c
     ka.dig_stride = w.dig_stride;
     ka.bstride = w.stride;
     ka.dig_bstride = hoisted ? 0 : w.stride;
-    launch_ks_inner(c->dev, level, nb, ka, false, w.st);
+    launch_ks_inner(c->dev, level, nb, ka, w.st);
     moddown_finish(c, w, level, nb, out0, out1, false, false);
 }
 
@@ -255,7 +239,7 @@ void eng_rotate_sum(fides_ctx* c, Workspace& w, int level, int nb, const uint64_
     ka.dig_stride = w.dig_stride;
     ka.bstride = w.stride;
     ka.dig_bstride = w.stride;
-    launch_ks_inner(c->dev, level, nb, ka, false, w.st);
+    launch_ks_inner(c->dev, level, nb, ka, w.st);
     ExtSumArgs sa{};
     sa.nout = nout;
     sa.n = level + 1;
@@ -269,7 +253,7 @@ void eng_rotate_sum(fides_ctx* c, Workspace& w, int level, int nb, const uint64_
     for (int u = 0; u < nout; ++u) {
         Workspace v = w;
         const size_t off = (size_t)start[u] * w.stride;
-        for (uint64_t** p : {&v.E0, &v.E1, &v.E2, &v.XT, &v.DIG, &v.XB, &v.XA, &v.W, &v.T}) *p += off;
+        for (uint64_t** p : {&v.XT, &v.DIG, &v.XB, &v.XA, &v.W, &v.T}) *p += off;
         moddown_finish(c, v, level, 1, out0 + u, out1 + u, false, false);
     }
 }
@@ -296,7 +280,7 @@ void eng_rotate_groups(fides_ctx* c, Workspace& w, int level, int ngroups, int n
     ka.bstride = w.stride;
     ka.dig_bstride = w.stride;
     ka.dig_group = nper;
-    launch_ks_inner(c->dev, level, nb, ka, false, w.st);
+    launch_ks_inner(c->dev, level, nb, ka, w.st);
     moddown_finish(c, w, level, nb, out0, out1, false, false);
 }
 

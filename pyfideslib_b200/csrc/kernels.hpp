@@ -12,12 +12,12 @@ enum { FL_PLAIN = 0, FL_SWITCHMOD = 1 };
 // forward-NTT epilogues (pass 2 stores); v = NTT value, j = prime, l = level
 enum {
     FS_PLAIN = 0,    // out = v
-    FS_MODDOWN = 1,  // out = (in2 - v) * P^-1 (+ in3)
+    FS_MODDOWN = 1,  // out = (in2 - v) * P^-1
     FS_RESCALE = 2,  // out = (in2 - v) * q_l^-1
-    FS_MDRS = 3,     // out = (in3 + in2 * P^-1 - v) * q_l^-1
+    FS_SUBP = 3,     // out = in2 - v * P^-1
 };
 // inverse-NTT prologues (pass A loads)
-enum { IL_PLAIN = 0, IL_MUL = 1, IL_AXPY_PINV = 2 };
+enum { IL_PLAIN = 0, IL_MUL = 1 };
 // inverse-NTT epilogues (pass B scale): N^-1 times 1 / ModUp hat-inverse / ModDown hat-inverse
 enum { IS_PLAIN = 0, IS_MODUP = 1, IS_MODDOWN = 2 };
 
@@ -51,12 +51,12 @@ uint64_t launch_count();
 void count_launches(int n);
 
 // the transforms of one ring dimension (ntt_n.cu)
-struct KsFuseArgs;
+struct KsHmultArgs;
 struct NttOps {
     void (*fwd)(const DevCtx&, const LimbMap&, cudaStream_t);
     void (*inv)(const DevCtx&, const LimbMap&, cudaStream_t);
     void (*fwd_cols)(const DevCtx&, const LimbMap&, cudaStream_t);
-    void (*rows_ks)(const DevCtx&, const KsFuseArgs&, int nb, cudaStream_t);
+    void (*rows_ks)(const DevCtx&, const KsHmultArgs&, int nb, cudaStream_t);
     void (*prepare)(const DevCtx&);
 };
 template <int LOGN>
@@ -78,26 +78,32 @@ void ntt_forward(const DevCtx& ctx, const LimbMap& map, int load, int store, cud
 void ntt_prepare(const DevCtx& ctx);
 // Forward NTT column pass alone (seg.in -> seg.out), for the fused key switch.
 void ntt_forward_cols(const DevCtx& ctx, const LimbMap& map, int load, cudaStream_t st);
-// Row pass of the ModUp digits fused with the key-switch inner product:
-//   XB[m] = sum_d D_d[t] kb[d][t],  XA[m] = sum_d D_d[t] ka[d][t]
-// over the extended basis m in [0, level+1+K) (prime t = m, or L + m - n for
-// the special limbs), for nb batch elements (blockIdx.y).  D_d[t] is the
-// column-pass output of digit d's limb in DIG, finished by the row stages
-// here, or the original evaluation limb `own` when t lies in digit d.
-struct KsFuseArgs {
-    const uint64_t* dig;  // ModUp digits of element 0 after the column pass
-    const uint64_t* own;  // key-switched polynomial in evaluation form, element 0
+// HMult's inner product with the rest of its tensor product, for nb batch
+// elements over the extended basis m in [0, level+1+K) (prime t = m, or
+// L + m - n for the special limbs):
+//   XB[m] = a0 b0 + P^-1 sum_d D_d[t] kb[d][t]
+//   XA[m] = a0 b1 + a1 b0 + P^-1 sum_d D_d[t] ka[d][t]     (m <= level)
+// and the bare sums for the special limbs.  D_d[t] is digit d's limb in DIG, or
+// the product a1 b1 when t lies in digit d.
+struct KsHmultArgs {
+    const uint64_t* a0[kMaxBatch];  // the elements' inputs (a0, a1), (b0, b1)
+    const uint64_t* a1[kMaxBatch];
+    const uint64_t* b0[kMaxBatch];
+    const uint64_t* b1[kMaxBatch];
+    const uint64_t* dig;  // ModUp digits of a1 b1, element 0 (fused kernel: after the column pass)
     const uint64_t* kb;   // switching key halves [dnum][L+K][N] (one key for the batch)
-    const uint64_t* ka;
+    const uint64_t* ka;   // null (not in the fused kernel): seeded, the a half regenerated from a_seed
+    uint64_t a_seed;      // uniform_stream(key seed, 0); digit d's stream is this ^ (d+1) << 48
     uint64_t* xb;         // outputs of element 0 [level+1+K][N]
     uint64_t* xa;
     size_t dig_stride;    // limbs per digit in dig
-    size_t bstride;       // words between consecutive elements of dig, own, xb, xa
+    size_t bstride;       // words between consecutive elements of dig, xb, xa
     int level;
-    int fp_sums;          // 1: exact FP64 sums for primes below 2^50
-    int m0;               // first output limb of a launch (set by the launcher)
+    int fp_sums;          // fused kernel: 1: exact FP64 sums for primes below 2^50
+    int nd, m0;           // set by the launcher: digits, first output limb
 };
-void ntt_rows_keyswitch(const DevCtx& ctx, const KsFuseArgs& a, int nb, cudaStream_t st);
+// its form fused into the digits' row pass (DIG after the column pass)
+void ntt_rows_keyswitch(const DevCtx& ctx, const KsHmultArgs& a, int nb, cudaStream_t st);
 // the fused row pass keeps one transformed tile per digit in shared memory
 bool ntt_rows_keyswitch_supported(const DevCtx& ctx);
 // Inverse NTT: pass A reads seg.in (+in2 for the prologue), writes seg.out;
@@ -107,17 +113,6 @@ void ntt_inverse(const DevCtx& ctx, const LimbMap& map, int load, int store, cud
 // ---- element-wise and base-conversion kernels (ks.cu) ----
 // Batched kernels take per-element pointers in kernel parameters (up to
 // kMaxBatch elements); workspace buffers of element b sit at ptr + b*bstride.
-struct TensorArgs {
-    const uint64_t* a0[kMaxBatch];
-    const uint64_t* a1[kMaxBatch];
-    const uint64_t* b0[kMaxBatch];
-    const uint64_t* b1[kMaxBatch];
-    uint64_t* e0;
-    uint64_t* e1;
-    uint64_t* e2;
-    size_t bstride;
-};
-void launch_tensor(const DevCtx& ctx, int n, int nb, const TensorArgs& args, cudaStream_t st);
 void launch_modup_conv(const DevCtx& ctx, int level, int nb, const uint64_t* xt, uint64_t* dig, size_t dig_stride,
                        size_t bstride, cudaStream_t st);
 struct KsArgs {
@@ -136,8 +131,9 @@ struct KsArgs {
     int dig_group;                   // > 0: element b reads the ModUp of element dig_elem[b] (grouped hoisting)
     uint8_t dig_elem[kMaxBatch];
 };
-// plain: no rotation in any element (vectorised variant)
-void launch_ks_inner(const DevCtx& ctx, int level, int nb, const KsArgs& args, bool plain, cudaStream_t st);
+void launch_ks_inner(const DevCtx& ctx, int level, int nb, const KsArgs& args, cudaStream_t st);
+// the inner product of a batch of products, with their tensor product
+void launch_ks_hmult(const DevCtx& ctx, int nb, const KsHmultArgs& args, cudaStream_t st);
 struct MdArgs {
     const uint64_t* y[2];     // scaled special limbs of the two halves (element 0)
     uint64_t* w[2];           // conversion outputs

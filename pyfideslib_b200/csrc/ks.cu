@@ -29,67 +29,6 @@ __device__ __forceinline__ uint32_t automorph_slot(int logN, uint32_t k, uint32_
 }
 
 // ---------------------------------------------------------------------------
-// tensor product (binomialMult_): e0 = a0 b0, e1 = a0 b1 + a1 b0, e2 = a1 b1,
-// for every batch element (blockIdx.z)
-// ---------------------------------------------------------------------------
-__global__ void k_tensor(const __grid_constant__ DevCtx ctx, const __grid_constant__ TensorArgs args) {
-    pdl_trigger();
-    pdl_wait();
-    const int limb = blockIdx.y, bi = blockIdx.z;
-    const PrimeConst pc = ctx.pc[limb];
-    const size_t i = ((size_t)limb * ctx.N + (size_t)(blockIdx.x * blockDim.x + threadIdx.x) * 2);
-    const size_t o = i + (size_t)bi * args.bstride;
-    const ulonglong2 x0 = *reinterpret_cast<const ulonglong2*>(args.a0[bi] + i);
-    const ulonglong2 x1 = *reinterpret_cast<const ulonglong2*>(args.a1[bi] + i);
-    const ulonglong2 y0 = *reinterpret_cast<const ulonglong2*>(args.b0[bi] + i);
-    const ulonglong2 y1 = *reinterpret_cast<const ulonglong2*>(args.b1[bi] + i);
-    ulonglong2 r0, r1, r2;
-    if (pc.p < kFpPrimeBound) {
-        // all three on the FP64 pipes (fp64.cuh: each product reduced to
-        // |r| <= 0.875p, e1's sum of two below 1.75p, then the floor
-        // reduction, exact for (-2p, 2p)): with 128-bit integer products the
-        // IMAD pipe, not HBM, bounds this kernel
-        const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
-        auto fmul = [&](uint64_t a, uint64_t b) {
-            return fp_to_u(fp_mulmod(as_f64(fp_from_u(a)), as_f64(fp_from_u(b)), p, pinv), p, pinv);
-        };
-        r0.x = fmul(x0.x, y0.x);
-        r0.y = fmul(x0.y, y0.y);
-        r2.x = fmul(x1.x, y1.x);
-        r2.y = fmul(x1.y, y1.y);
-        auto fsum = [&](uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
-            const double s = __dadd_rn(fp_mulmod(as_f64(fp_from_u(a)), as_f64(fp_from_u(b)), p, pinv),
-                                       fp_mulmod(as_f64(fp_from_u(c)), as_f64(fp_from_u(d)), p, pinv));
-            return fp_to_u(s, p, pinv);
-        };
-        r1.x = fsum(x0.x, y1.x, x1.x, y0.x);
-        r1.y = fsum(x0.y, y1.y, x1.y, y0.y);
-    } else {
-        r0.x = mul_mod(x0.x, y0.x, pc);
-        r0.y = mul_mod(x0.y, y0.y, pc);
-        r2.x = mul_mod(x1.x, y1.x, pc);
-        r2.y = mul_mod(x1.y, y1.y, pc);
-        Acc128 s;
-        s.mac(x0.x, y1.x);
-        s.mac(x1.x, y0.x);
-        r1.x = s.reduce(pc);
-        Acc128 t;
-        t.mac(x0.y, y1.y);
-        t.mac(x1.y, y0.y);
-        r1.y = t.reduce(pc);
-    }
-    *reinterpret_cast<ulonglong2*>(args.e0 + o) = r0;
-    *reinterpret_cast<ulonglong2*>(args.e1 + o) = r1;
-    *reinterpret_cast<ulonglong2*>(args.e2 + o) = r2;
-}
-
-void launch_tensor(const DevCtx& ctx, int n, int nb, const TensorArgs& args, cudaStream_t st) {
-    dim3 g(ctx.N / 256, n, nb);
-    count_launches(1);
-    launch_pdl(k_tensor, g, 128, 0, st, ctx, args);
-}
-
-// ---------------------------------------------------------------------------
 // ModUp base conversion (DecompAndModUpConv): for digit d at `level`, with
 // inputs xt_i = [x_i * (Q'/q_i)^-1]_{q_i} (produced by the scaled INTT), every
 // target prime t outside the digit gets  sum_i xt_i * [Q'/q_i]_t  mod t.
@@ -282,9 +221,10 @@ void launch_modup_conv(const DevCtx& ctx, int level, int nb, const uint64_t* xt,
 // k'_d[j] = k_d[slot(g, j)] (the key that switches sigma_g(s) back to s):
 // only the digit values and c0 are gathered, the key streams in order.
 // ---------------------------------------------------------------------------
-// Batch element b = blockIdx.x % nb varies fastest, so the blocks that read
-// one key tile for the different elements run back to back and the key is
-// fetched from HBM once and served from L2 to the rest of the batch.
+// The batch elements of one limb run one after the other (blockIdx.y), so the
+// key limb (or hoisted digits) they share is fetched from HBM once and served
+// from L2 to the rest of the batch.  (Folding the element into blockIdx.x and
+// dividing by the batch size per thread cost 32 hoisted rotations 1.1%.)
 // FPK: limbs of primes below 2^50 accumulate on the FP64 pipes (fp64.cuh):
 // each product x k is reduced to |r| <= 0.875p, the sum of up to 8 digits
 // stays below 7p < 2^53, and one centring plus a floor reduction give the
@@ -300,18 +240,17 @@ constexpr bool kIsSplitAcc = false;
 template <>
 constexpr bool kIsSplitAcc<AccSplit> = true;
 
-template <int VEC, class ACC, bool FPK, bool GRP = false, bool SEED = false>
+template <class ACC, bool FPK, bool GRP, bool SEED>
 __global__ void __launch_bounds__(256, SEED ? (FPK ? 5 : (kIsSplitAcc<ACC> ? 0 : 6)) : 0)
-    k_ks_inner(const __grid_constant__ DevCtx ctx, int level, int nb, const __grid_constant__ KsArgs args) {
+    k_ks_inner(const __grid_constant__ DevCtx ctx, int level, int nd, const __grid_constant__ KsArgs args) {
     pdl_trigger();
     pdl_wait();
     const int n = level + 1;
-    const int m = blockIdx.y;
-    const int bi = blockIdx.x % nb;
-    const int bx = blockIdx.x / nb;
+    const int m = blockIdx.z;
+    const int bi = blockIdx.y;
+    const int bx = blockIdx.x;
     const int t = m < n ? m : ctx.L + (m - n);
     const PrimeConst pc = ctx.pc[t];
-    const int nd = level / ctx.alpha + 1;
     const size_t kstride = (size_t)(ctx.L + ctx.K) * ctx.N;
     const size_t boff = (size_t)bi * args.bstride;
     const uint64_t* kb = args.kb[bi];
@@ -337,69 +276,7 @@ __global__ void __launch_bounds__(256, SEED ? (FPK ? 5 : (kIsSplitAcc<ACC> ? 0 :
     }
     uint64_t* xb = args.xb + boff + (size_t)m * ctx.N;
     uint64_t* xa = args.xa + boff + (size_t)m * ctx.N;
-    if constexpr (VEC && FPK) {
-        if (pc.p < kFpPrimeBound) {
-            const size_t j = ((size_t)bx * blockDim.x + threadIdx.x) * 2;
-            const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
-            double sb0 = 0, sb1 = 0, sa0 = 0, sa1 = 0;
-#pragma unroll
-            for (int d = 0; d < 8; ++d) {
-                if (d < nd) {
-                    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(srcs[d] + j);
-                    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(kb + d * kstride + (size_t)t * ctx.N + j);
-                    ulonglong2 a;
-                    if (!SEED || ka) {
-                        a = *reinterpret_cast<const ulonglong2*>(ka + d * kstride + (size_t)t * ctx.N + j);
-                    } else {
-                        a.x = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j, pc.p);
-                        a.y = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j + 1, pc.p);
-                    }
-                    const double x0 = as_f64(fp_from_u(x.x)), x1 = as_f64(fp_from_u(x.y));
-                    sb0 = __dadd_rn(sb0, fp_mulmod(x0, as_f64(fp_from_u(b.x)), p, pinv));
-                    sb1 = __dadd_rn(sb1, fp_mulmod(x1, as_f64(fp_from_u(b.y)), p, pinv));
-                    sa0 = __dadd_rn(sa0, fp_mulmod(x0, as_f64(fp_from_u(a.x)), p, pinv));
-                    sa1 = __dadd_rn(sa1, fp_mulmod(x1, as_f64(fp_from_u(a.y)), p, pinv));
-                }
-            }
-            ulonglong2 ob, oa;
-            ob.x = fp_sum_to_u(sb0, p, pinv);
-            ob.y = fp_sum_to_u(sb1, p, pinv);
-            oa.x = fp_sum_to_u(sa0, p, pinv);
-            oa.y = fp_sum_to_u(sa1, p, pinv);
-            *reinterpret_cast<ulonglong2*>(xb + j) = ob;
-            *reinterpret_cast<ulonglong2*>(xa + j) = oa;
-            return;
-        }
-    }
-    if constexpr (VEC) {
-        const size_t j = ((size_t)bx * blockDim.x + threadIdx.x) * 2;
-        ACC sb0, sb1, sa0, sa1;
-#pragma unroll
-        for (int d = 0; d < 8; ++d) {
-            if (d < nd) {
-                const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(srcs[d] + j);
-                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(kb + d * kstride + (size_t)t * ctx.N + j);
-                ulonglong2 a;
-                if (!SEED || ka) {
-                    a = *reinterpret_cast<const ulonglong2*>(ka + d * kstride + (size_t)t * ctx.N + j);
-                } else {
-                    a.x = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j, pc.p);
-                    a.y = uniform_mod(astream ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j + 1, pc.p);
-                }
-                sb0.mac(x.x, b.x);
-                sb1.mac(x.y, b.y);
-                sa0.mac(x.x, a.x);
-                sa1.mac(x.y, a.y);
-            }
-        }
-        ulonglong2 ob, oa;
-        ob.x = sb0.reduce(pc);
-        ob.y = sb1.reduce(pc);
-        oa.x = sa0.reduce(pc);
-        oa.y = sa1.reduce(pc);
-        *reinterpret_cast<ulonglong2*>(xb + j) = ob;
-        *reinterpret_cast<ulonglong2*>(xa + j) = oa;
-    } else {
+    {
         // rotation: outputs j, j+1 gather the digit values (and c0) at the
         // automorphism's source slots; the key is stored permuted (entry j is
         // the one that pairs with output j), so its loads stay vectorised.
@@ -493,42 +370,185 @@ __global__ void __launch_bounds__(256, SEED ? (FPK ? 5 : (kIsSplitAcc<ACC> ? 0 :
     }
 }
 
-template <int VEC, class ACC, bool FPK, bool GRP>
-static void ks_inner_go(const DevCtx& ctx, int level, int nb, const KsArgs& args, bool seeded, dim3 g,
+template <class ACC, bool FPK, bool GRP>
+static void ks_inner_go(const DevCtx& ctx, int level, int nd, const KsArgs& args, bool seeded, dim3 g,
                         cudaStream_t st) {
     if (seeded)
-        launch_pdl(k_ks_inner<VEC, ACC, FPK, GRP, true>, g, 256, 0, st, ctx, level, nb, args);
+        launch_pdl(k_ks_inner<ACC, FPK, GRP, true>, g, 256, 0, st, ctx, level, nd, args);
     else
-        launch_pdl(k_ks_inner<VEC, ACC, FPK, GRP, false>, g, 256, 0, st, ctx, level, nb, args);
+        launch_pdl(k_ks_inner<ACC, FPK, GRP, false>, g, 256, 0, st, ctx, level, nd, args);
 }
 
-void launch_ks_inner(const DevCtx& ctx, int level, int nb, const KsArgs& args, bool plain, cudaStream_t st) {
+void launch_ks_inner(const DevCtx& ctx, int level, int nb, const KsArgs& args, cudaStream_t st) {
     count_launches(1);
     bool seeded = false;
     for (int b = 0; b < nb; ++b) seeded = seeded || args.ka[b] == nullptr;
-    if (plain) {
-        dim3 g(ctx.N / 512 * nb, level + 1 + ctx.K);
+    const int nd = level / ctx.alpha + 1;
+    const dim3 g(ctx.N / 512, nb, level + 1 + ctx.K);
+    if (args.dig_group > 0) {
         if (ctx.ks_variant & 1)
-            ks_inner_go<1, Acc128, true, false>(ctx, level, nb, args, seeded, g, st);
-        else if (ctx.conv_variant == 1)
-            ks_inner_go<1, AccSplit, false, false>(ctx, level, nb, args, seeded, g, st);
+            ks_inner_go<Acc128, true, true>(ctx, level, nd, args, seeded, g, st);
         else
-            ks_inner_go<1, Acc128, false, false>(ctx, level, nb, args, seeded, g, st);
-    } else if (args.dig_group > 0) {
-        dim3 g(ctx.N / 512 * nb, level + 1 + ctx.K);
-        if (ctx.ks_variant & 1)
-            ks_inner_go<0, Acc128, true, true>(ctx, level, nb, args, seeded, g, st);
-        else
-            ks_inner_go<0, Acc128, false, true>(ctx, level, nb, args, seeded, g, st);
+            ks_inner_go<Acc128, false, true>(ctx, level, nd, args, seeded, g, st);
     } else {
-        dim3 g(ctx.N / 512 * nb, level + 1 + ctx.K);
         if (ctx.ks_variant & 1)
-            ks_inner_go<0, Acc128, true, false>(ctx, level, nb, args, seeded, g, st);
+            ks_inner_go<Acc128, true, false>(ctx, level, nd, args, seeded, g, st);
         else if (ctx.conv_variant == 1)
-            ks_inner_go<0, AccSplit, false, false>(ctx, level, nb, args, seeded, g, st);
+            ks_inner_go<AccSplit, false, false>(ctx, level, nd, args, seeded, g, st);
         else
-            ks_inner_go<0, Acc128, false, false>(ctx, level, nb, args, seeded, g, st);
+            ks_inner_go<Acc128, false, false>(ctx, level, nd, args, seeded, g, st);
     }
+}
+
+// ---------------------------------------------------------------------------
+// key-switch inner product of a product (a0, a1)(b0, b1), with the tensor
+// product (binomialMult_) formed on the way: the own limb of digit d is a1 b1,
+// and the ciphertext limbs leave as e + P^-1 x,
+//   XB[m] = a0 b0 + P^-1 sum_d D_d[t] kb[d][t]
+//   XA[m] = a0 b1 + a1 b0 + P^-1 sum_d D_d[t] ka[d][t]      (m < n),
+// the special limbs as the sums.  Bounds and sums as in k_ks_inner.
+// ---------------------------------------------------------------------------
+// HBM bounds this kernel in a batch, its loads' latency in a single product.
+// ModUp's inverse transform takes a1 b1 in its own load, so no limb of the
+// tensor product is stored: 8 limbs of traffic per limb of the level instead of
+// 13 around the tensor product, that inverse, this kernel and the final row
+// pass, and one launch less.  64 registers: 4 CTAs per SM, without spills (left
+// free it takes 72, 3 CTAs, one product at N = 2^16 258 us instead of 251).
+// N = 2^16, L = 30, with a tensor kernel / this: one product 260 / 251 us, 21
+// pairs at uneven levels 6449 / 6122 us.  Large batches form these sums in the
+// epilogue of the digits' row pass instead (k_ntt_fwd_rows_ks).
+template <bool FPK, bool SEED>
+__global__ void __launch_bounds__(256, 4)
+    k_ks_hmult(const __grid_constant__ DevCtx ctx, const __grid_constant__ KsHmultArgs args) {
+    pdl_trigger();
+    pdl_wait();
+    const int n = args.level + 1, nd = args.nd;
+    const int m = blockIdx.z;
+    const int bi = blockIdx.y;  // a limb's elements run together and share its key tiles through L2
+    const bool tensor = m < n;
+    const int t = tensor ? m : ctx.L + (m - n);
+    const PrimeConst pc = ctx.pc[t];
+    const size_t kstride = (size_t)(ctx.L + ctx.K) * ctx.N;
+    const size_t boff = (size_t)bi * args.bstride;
+    const size_t j = ((size_t)blockIdx.x * 256 + threadIdx.x) * 2;
+    const size_t koff = (size_t)t * ctx.N + j;
+    auto word = [&](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q + koff); };
+    auto own_digit = [&](int d) { return tensor && (unsigned)(m - d * ctx.alpha) < (unsigned)ctx.alpha; };
+    auto digit = [&](int d) {  // ModUp output of digit d: the Q primes outside it, then the special primes
+        const int lo = d * ctx.alpha, cnt = min(ctx.alpha, n - lo);
+        return *reinterpret_cast<const ulonglong2*>(
+            args.dig + boff + ((size_t)d * args.dig_stride + (m < lo ? m : m - cnt)) * ctx.N + j);
+    };
+    auto key_a = [&](int d) {
+        ulonglong2 a;
+        if (!SEED) {
+            a = word(args.ka + d * kstride);
+        } else {
+            a.x = uniform_mod(args.a_seed ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j, pc.p);
+            a.y = uniform_mod(args.a_seed ^ ((uint64_t)(d + 1) << 48), t, (uint32_t)j + 1, pc.p);
+        }
+        return a;
+    };
+    ulonglong2 a0, a1, b0, b1;
+    if (tensor) {
+        a0 = word(args.a0[bi]);
+        a1 = word(args.a1[bi]);
+        b0 = word(args.b0[bi]);
+        b1 = word(args.b1[bi]);
+    }
+    ulonglong2 ob, oa;
+    if (FPK && pc.p < kFpPrimeBound) {
+        const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
+        auto conv = [](uint64_t u) { return as_f64(fp_from_u(u)); };
+        auto prod = [&](uint64_t u, uint64_t v) { return fp_mulmod(conv(u), conv(v), p, pinv); };
+        double sb0 = 0, sb1 = 0, sa0 = 0, sa1 = 0;
+#pragma unroll
+        for (int d = 0; d < 8; ++d) {
+            if (d < nd) {
+                const ulonglong2 b = word(args.kb + d * kstride), a = key_a(d);
+                double x0, x1;
+                if (own_digit(d)) {
+                    x0 = prod(a1.x, b1.x);
+                    x1 = prod(a1.y, b1.y);
+                } else {
+                    const ulonglong2 x = digit(d);
+                    x0 = conv(x.x);
+                    x1 = conv(x.y);
+                }
+                sb0 = __dadd_rn(sb0, fp_mulmod(x0, conv(b.x), p, pinv));
+                sb1 = __dadd_rn(sb1, fp_mulmod(x1, conv(b.y), p, pinv));
+                sa0 = __dadd_rn(sa0, fp_mulmod(x0, conv(a.x), p, pinv));
+                sa1 = __dadd_rn(sa1, fp_mulmod(x1, conv(a.y), p, pinv));
+            }
+        }
+        if (tensor) {
+            // P^-1 times the centred sum (< 0.54p) plus one or two products (<= 0.875p each)
+            const double2 ci = __ldg(reinterpret_cast<const double2*>(ctx.md_pinvf) + t);
+            auto down = [&](double s) { return fp_mulw(fp_center(s, p, pinv), ci.x, ci.y, p); };
+            sb0 = __dadd_rn(down(sb0), prod(a0.x, b0.x));
+            sb1 = __dadd_rn(down(sb1), prod(a0.y, b0.y));
+            sa0 = __dadd_rn(__dadd_rn(down(sa0), prod(a0.x, b1.x)), prod(a1.x, b0.x));
+            sa1 = __dadd_rn(__dadd_rn(down(sa1), prod(a0.y, b1.y)), prod(a1.y, b0.y));
+        }
+        ob.x = fp_sum_to_u(sb0, p, pinv);
+        ob.y = fp_sum_to_u(sb1, p, pinv);
+        oa.x = fp_sum_to_u(sa0, p, pinv);
+        oa.y = fp_sum_to_u(sa1, p, pinv);
+    } else {
+        Acc128 sb0, sb1, sa0, sa1;
+#pragma unroll
+        for (int d = 0; d < 8; ++d) {
+            if (d < nd) {
+                const ulonglong2 b = word(args.kb + d * kstride), a = key_a(d);
+                const ulonglong2 x = own_digit(d) ? make_ulonglong2(mul_mod(a1.x, b1.x, pc), mul_mod(a1.y, b1.y, pc))
+                                                  : digit(d);
+                sb0.mac(x.x, b.x);
+                sb1.mac(x.y, b.y);
+                sa0.mac(x.x, a.x);
+                sa1.mac(x.y, a.y);
+            }
+        }
+        ob.x = sb0.reduce(pc);
+        ob.y = sb1.reduce(pc);
+        oa.x = sa0.reduce(pc);
+        oa.y = sa1.reduce(pc);
+        if (tensor) {
+            const ulonglong2 ci = __ldg(reinterpret_cast<const ulonglong2*>(ctx.md_pinv) + t);
+            auto cross = [&](uint64_t u0, uint64_t v0, uint64_t u1, uint64_t v1) {
+                Acc128 e;
+                e.mac(u0, v0);
+                e.mac(u1, v1);
+                return e.reduce(pc);
+            };
+            auto down = [&](uint64_t s, uint64_t e) { return add_mod(mul_shoup(s, ci.x, ci.y, pc.p), e, pc.p); };
+            ob.x = down(ob.x, mul_mod(a0.x, b0.x, pc));
+            ob.y = down(ob.y, mul_mod(a0.y, b0.y, pc));
+            oa.x = down(oa.x, cross(a0.x, b1.x, a1.x, b0.x));
+            oa.y = down(oa.y, cross(a0.y, b1.y, a1.y, b0.y));
+        }
+    }
+    const size_t o = boff + (size_t)m * ctx.N + j;
+    *reinterpret_cast<ulonglong2*>(args.xb + o) = ob;
+    *reinterpret_cast<ulonglong2*>(args.xa + o) = oa;
+}
+
+template <bool FPK>
+static void ks_hmult_go(const DevCtx& ctx, int nb, const KsHmultArgs& args, cudaStream_t st) {
+    const dim3 g(ctx.N / 512, nb, args.level + 1 + ctx.K);
+    if (args.ka == nullptr)
+        launch_pdl(k_ks_hmult<FPK, true>, g, 256, 0, st, ctx, args);
+    else
+        launch_pdl(k_ks_hmult<FPK, false>, g, 256, 0, st, ctx, args);
+}
+
+void launch_ks_hmult(const DevCtx& ctx, int nb, const KsHmultArgs& a, cudaStream_t st) {
+    count_launches(1);
+    KsHmultArgs args = a;
+    args.nd = a.level / ctx.alpha + 1;
+    if (ctx.ks_variant & 1)
+        ks_hmult_go<true>(ctx, nb, args, st);
+    else
+        ks_hmult_go<false>(ctx, nb, args, st);
 }
 
 // ---------------------------------------------------------------------------

@@ -77,7 +77,7 @@ void ntt_forward_cols(const DevCtx& ctx, const LimbMap& m, int load, cudaStream_
     ops_of(ctx.logN)->fwd_cols(ctx, map, st);
 }
 
-void ntt_rows_keyswitch(const DevCtx& ctx, const KsFuseArgs& a, int nb, cudaStream_t st) {
+void ntt_rows_keyswitch(const DevCtx& ctx, const KsHmultArgs& a, int nb, cudaStream_t st) {
     count_launches(1);
     ops_of(ctx.logN)->rows_ks(ctx, a, nb, st);
 }

@@ -408,20 +408,19 @@ struct RowFwd {
     }
 };
 
-// The epilogue of one warp's tile: out[i] = f(value, in2[i], in3[i]) over the
+// The epilogue of one warp's tile: out[i] = f(value, in2[i]) over the
 // words of the tile, two adjacent words per lane and step (16-byte accesses).
-// NIN: operands read (in3 may be null: reads as 0).
-template <class G, int NIN, class F>
+// IN2: whether in2 is read (else 0).
+template <class G, bool IN2, class F>
 __device__ __forceinline__ void row_epilogue(const LimbRef& lr, size_t base, const uint64_t* sw, int lane, F f) {
 #pragma unroll 4
     for (int j = 0; j < 8; ++j) {
         const int i = 2 * lane + 2 * G::WL * j;
         const int wi = padi(i);
-        ulonglong2 a = make_ulonglong2(0, 0), b = a, o;
-        if (NIN > 0) a = *reinterpret_cast<const ulonglong2*>(lr.in2 + base + i);
-        if (NIN > 1 && lr.in3) b = *reinterpret_cast<const ulonglong2*>(lr.in3 + base + i);
-        o.x = f(sw[wi], a.x, b.x);
-        o.y = f(sw[wi + 1], a.y, b.y);
+        ulonglong2 a = make_ulonglong2(0, 0), o;
+        if (IN2) a = *reinterpret_cast<const ulonglong2*>(lr.in2 + base + i);
+        o.x = f(sw[wi], a.x);
+        o.y = f(sw[wi + 1], a.y);
         *reinterpret_cast<ulonglong2*>(lr.out + base + i) = o;
     }
 }
@@ -454,13 +453,12 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
 #pragma unroll
     for (int k = 0; k < 16; ++k) x[k] = src[th + (k << (LC - 4))];
     if (lr.smode != FS_PLAIN && lr.in2 && gridDim.y > 1) {
-        // the epilogue's operands for this tile (one 128-byte line per lane
-        // and operand): start their HBM reads now, under the butterflies.
+        // the epilogue's operand for this tile (one 128-byte line per lane):
+        // start its HBM reads now, under the butterflies.
         // Batched launches only: a single element's grid is about two waves,
         // where the early reads only compete with the row loads (measured
         // 1.5% slower per operation, 0.5% faster batched)
         prefetch_l2(lr.in2 + base + lane * 16);
-        if (lr.in3) prefetch_l2(lr.in3 + base + lane * 16);
     }
     stage_wait();
     __syncwarp(G::MASK);
@@ -481,50 +479,36 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
         // every product is below 0.62p and the last one, shifted by p, is
         // positive.  (64-bit Shoup products here cost as many issue slots as the
         // butterflies: the final row pass of 32 products took 925 us, 58 x 32 limbs.)
-        const double2 ci = lr.smode == FS_PLAIN || lr.smode == FS_RESCALE
-                               ? make_double2(0, 0)
-                               : *reinterpret_cast<const double2*>(ctx.md_pinvf + 2 * lr.prime);
-        const double2 cq = lr.smode == FS_RESCALE || lr.smode == FS_MDRS
-                               ? *reinterpret_cast<const double2*>(ctx.rs_qinvf + 2 * ((size_t)lr.level * ctx.L + lr.prime))
-                               : make_double2(0, 0);
+        const double2 c = lr.smode == FS_PLAIN ? make_double2(0, 0)
+                          : lr.smode == FS_RESCALE
+                              ? *reinterpret_cast<const double2*>(ctx.rs_qinvf + 2 * ((size_t)lr.level * ctx.L + lr.prime))
+                              : *reinterpret_cast<const double2*>(ctx.md_pinvf + 2 * lr.prime);
         auto conv = [](uint64_t u) { return as_f64(fp_from_u(u)); };
         if (lr.smode == FS_PLAIN)
-            row_epilogue<G, 0>(lr, base, sw, lane,
-                               [&](uint64_t v, uint64_t, uint64_t) { return fp_pos_to_u(as_f64(v), p, pinv); });
-        else if (lr.smode == FS_MODDOWN)
-            row_epilogue<G, 2>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t b) {
-                const double t = fp_mulw_sh(__dsub_rn(conv(a), as_f64(v)), ci.x, ci.y, p, kRint + 1.0);
-                return fp_pos_to_u(__dadd_rn(t, conv(b)), p, pinv);
-            });
-        else if (lr.smode == FS_RESCALE)
-            row_epilogue<G, 1>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t) {
-                return fp_pos_to_u(fp_mulw_sh(__dsub_rn(conv(a), as_f64(v)), cq.x, cq.y, p, kRint + 1.0), p, pinv);
+            row_epilogue<G, false>(lr, base, sw, lane,
+                                   [&](uint64_t v, uint64_t) { return fp_pos_to_u(as_f64(v), p, pinv); });
+        else if (lr.smode == FS_SUBP)
+            row_epilogue<G, true>(lr, base, sw, lane, [&](uint64_t v, uint64_t a) {
+                return fp_pos_to_u(__dadd_rn(conv(a), fp_mulw_sh(-as_f64(v), c.x, c.y, p, kRint + 1.0)), p, pinv);
             });
         else
-            row_epilogue<G, 2>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t b) {
-                const double u = __dadd_rn(conv(b), fp_mulw(conv(a), ci.x, ci.y, p));
-                return fp_pos_to_u(fp_mulw_sh(__dsub_rn(u, as_f64(v)), cq.x, cq.y, p, kRint + 1.0), p, pinv);
+            row_epilogue<G, true>(lr, base, sw, lane, [&](uint64_t v, uint64_t a) {
+                return fp_pos_to_u(fp_mulw_sh(__dsub_rn(conv(a), as_f64(v)), c.x, c.y, p, kRint + 1.0), p, pinv);
             });
         return;
     }
-    const ulonglong2 ci = lr.smode == FS_PLAIN || lr.smode == FS_RESCALE ? make_ulonglong2(0, 0) : ldg2(ctx.md_pinv, lr.prime);
-    const ulonglong2 cq = lr.smode == FS_RESCALE || lr.smode == FS_MDRS
-                              ? ldg2(ctx.rs_qinv, (size_t)lr.level * ctx.L + lr.prime)
-                              : make_ulonglong2(0, 0);
+    const ulonglong2 c = lr.smode == FS_PLAIN ? make_ulonglong2(0, 0)
+                         : lr.smode == FS_RESCALE ? ldg2(ctx.rs_qinv, (size_t)lr.level * ctx.L + lr.prime)
+                                                  : ldg2(ctx.md_pinv, lr.prime);
     if (lr.smode == FS_PLAIN)
-        row_epilogue<G, 0>(lr, base, sw, lane, [&](uint64_t v, uint64_t, uint64_t) { return reduce_fwd(v, pc); });
-    else if (lr.smode == FS_MODDOWN)
-        row_epilogue<G, 2>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t b) {
-            return add_mod(mul_shoup(sub_mod(a, reduce_fwd(v, pc), pc.p), ci.x, ci.y, pc.p), b, pc.p);
-        });
-    else if (lr.smode == FS_RESCALE)
-        row_epilogue<G, 1>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t) {
-            return mul_shoup(sub_mod(a, reduce_fwd(v, pc), pc.p), cq.x, cq.y, pc.p);
+        row_epilogue<G, false>(lr, base, sw, lane, [&](uint64_t v, uint64_t) { return reduce_fwd(v, pc); });
+    else if (lr.smode == FS_SUBP)
+        row_epilogue<G, true>(lr, base, sw, lane, [&](uint64_t v, uint64_t a) {
+            return sub_mod(a, mul_shoup(reduce_fwd(v, pc), c.x, c.y, pc.p), pc.p);
         });
     else
-        row_epilogue<G, 2>(lr, base, sw, lane, [&](uint64_t v, uint64_t a, uint64_t b) {
-            const uint64_t u = add_mod(b, mul_shoup(a, ci.x, ci.y, pc.p), pc.p);
-            return mul_shoup(sub_mod(u, reduce_fwd(v, pc), pc.p), cq.x, cq.y, pc.p);
+        row_epilogue<G, true>(lr, base, sw, lane, [&](uint64_t v, uint64_t a) {
+            return mul_shoup(sub_mod(a, reduce_fwd(v, pc), pc.p), c.x, c.y, pc.p);
         });
 }
 
@@ -544,6 +528,10 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
 // products fused into the NTT epilogue, ksk_dot_fusion / ksk_dot_acc_fusion
 // (src/NTTfusions.cuh:295-345) in the KSK_DOT modes of NTT_ (src/NTT.cu:680-700).
 //
+// The own limb is the product a1 b1 of the element's inputs, formed here, and
+// the ciphertext limbs' epilogue adds the rest of the tensor product, as in
+// k_ks_hmult.
+//
 // Sums: for primes below 2^50 with fp_sums, each product is an exact FP64
 // fp_mulmod of a transformed value (below 1.7p: the last row stage centres) or
 // the own limb (< p) with a key residue (< p): |r| <= (1/2 + 1.7 * 3/8) p, and
@@ -560,7 +548,7 @@ constexpr size_t ks_warp_words(int tiles) {
 
 template <int LR, int LC, bool FP, int MB>
 __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
-    k_ntt_fwd_rows_ks(const __grid_constant__ DevCtx ctx, const __grid_constant__ KsFuseArgs a, int tiles) {
+    k_ntt_fwd_rows_ks(const __grid_constant__ DevCtx ctx, const __grid_constant__ KsHmultArgs a, int tiles) {
     using G = RowGeo<LR, LC>;
     extern __shared__ __align__(16) uint64_t ks_sm[];  // per warp: twiddles, then one tile per digit needing rows
 
@@ -579,8 +567,10 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
     const size_t base = (size_t)row0 * G::C;
     const size_t kstride = (size_t)(ctx.L + ctx.K) * ctx.N;
     const size_t limb_off = (size_t)t * ctx.N + base;
-    const int nd = level / ctx.alpha + 1;
-    const int d_own = m < n ? t / ctx.alpha : -1;  // digit holding t (its value is the own limb)
+    const int nd = a.nd;
+    int d_own = -1;  // digit holding t (its value is the own limb)
+    for (int d = 0; d < nd; ++d)
+        if (m < n && (unsigned)(t - d * ctx.alpha) < (unsigned)ctx.alpha) d_own = d;
     uint64_t* wsm = ks_sm + (size_t)w * ks_warp_words<LR, LC>(tiles);
     ulonglong2* s_tw = reinterpret_cast<ulonglong2*>(wsm);
     uint64_t* s_tile = wsm + 2 * G::TW;
@@ -595,7 +585,14 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
         prefetch_l2(a.ka + d * kstride + limb_off + lane * 16);
     }
     pdl_wait();
-    if (d_own >= 0) prefetch_l2(a.own + boff + limb_off + lane * 16);
+    const bool tensor = m < n;
+    const int bi = blockIdx.y;
+    if (tensor) {
+        prefetch_l2(a.a0[bi] + limb_off + lane * 16);
+        prefetch_l2(a.a1[bi] + limb_off + lane * 16);
+        prefetch_l2(a.b0[bi] + limb_off + lane * 16);
+        prefetch_l2(a.b1[bi] + limb_off + lane * 16);
+    }
     stage_wait();
     __syncwarp(G::MASK);
 
@@ -624,11 +621,21 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
     const bool fpk = a.fp_sums && pc.p < kFpPrimeBound;
     uint64_t* xb = a.xb + boff + (size_t)m * ctx.N + base;
     uint64_t* xa = a.xa + boff + (size_t)m * ctx.N + base;
+    auto word = [&](const uint64_t* q, int i) { return *reinterpret_cast<const ulonglong2*>(q + limb_off + i); };
     for (int i = 2 * lane; i < G::GW; i += 2 * G::WL) {
         const int wi = padi(i);
         ulonglong2 ob, oa;
+        ulonglong2 ta0, ta1, tb0, tb1;  // the inputs of the tensor product
+        if (tensor) {
+            ta0 = word(a.a0[bi], i);
+            ta1 = word(a.a1[bi], i);
+            tb0 = word(a.b0[bi], i);
+            tb1 = word(a.b1[bi], i);
+        }
         if (fpk) {
             double sb0 = 0, sb1 = 0, sa0 = 0, sa1 = 0;
+            auto conv = [](uint64_t u) { return as_f64(fp_from_u(u)); };
+            auto prod = [&](uint64_t u, uint64_t v) { return fp_mulmod(conv(u), conv(v), p, pinv); };
 #pragma unroll
             for (int d = 0; d < 6; ++d) {
                 if (d < nd) {
@@ -636,9 +643,8 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
                     const ulonglong2 ka2 = *reinterpret_cast<const ulonglong2*>(a.ka + d * kstride + limb_off + i);
                     double x0, x1;
                     if (d == d_own) {
-                        const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(a.own + boff + limb_off + i);
-                        x0 = as_f64(fp_from_u(o.x));
-                        x1 = as_f64(fp_from_u(o.y));
+                        x0 = prod(ta1.x, tb1.x);
+                        x1 = prod(ta1.y, tb1.y);
                     } else {
                         const uint64_t* tile = s_tile + (size_t)(d_own >= 0 && d > d_own ? d - 1 : d) * G::SW;
                         if (fp) {
@@ -655,6 +661,16 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
                     sa1 = __dadd_rn(sa1, fp_mulmod(x1, as_f64(fp_from_u(ka2.y)), p, pinv));
                 }
             }
+            if (tensor) {
+                // P^-1 times the centred sum (< 0.54p) plus one or two products
+                // (<= 0.875p each)
+                const double2 ci = *reinterpret_cast<const double2*>(ctx.md_pinvf + 2 * t);
+                auto down = [&](double s) { return fp_mulw(fp_center(s, p, pinv), ci.x, ci.y, p); };
+                sb0 = __dadd_rn(down(sb0), prod(ta0.x, tb0.x));
+                sb1 = __dadd_rn(down(sb1), prod(ta0.y, tb0.y));
+                sa0 = __dadd_rn(__dadd_rn(down(sa0), prod(ta0.x, tb1.x)), prod(ta1.x, tb0.x));
+                sa1 = __dadd_rn(__dadd_rn(down(sa1), prod(ta0.y, tb1.y)), prod(ta1.y, tb0.y));
+            }
             ob.x = fp_sum_to_u(sb0, p, pinv);
             ob.y = fp_sum_to_u(sb1, p, pinv);
             oa.x = fp_sum_to_u(sa0, p, pinv);
@@ -668,9 +684,8 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
                     const ulonglong2 ka2 = *reinterpret_cast<const ulonglong2*>(a.ka + d * kstride + limb_off + i);
                     uint64_t x0, x1;
                     if (d == d_own) {
-                        const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(a.own + boff + limb_off + i);
-                        x0 = o.x;
-                        x1 = o.y;
+                        x0 = mul_mod(ta1.x, tb1.x, pc);
+                        x1 = mul_mod(ta1.y, tb1.y, pc);
                     } else {
                         const uint64_t* tile = s_tile + (size_t)(d_own >= 0 && d > d_own ? d - 1 : d) * G::SW;
                         if (fp) {
@@ -691,6 +706,19 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
             ob.y = sb1.reduce(pc);
             oa.x = sa0.reduce(pc);
             oa.y = sa1.reduce(pc);
+            if (tensor) {
+                const ulonglong2 ci = ldg2(ctx.md_pinv, t);
+                auto sum = [&](uint64_t s, uint64_t u0, uint64_t v0, uint64_t u1, uint64_t v1) {
+                    Acc128 e;
+                    e.mac(u0, v0);
+                    e.mac(u1, v1);
+                    return add_mod(mul_shoup(s, ci.x, ci.y, pc.p), e.reduce(pc), pc.p);
+                };
+                ob.x = sum(ob.x, ta0.x, tb0.x, 0, 0);
+                ob.y = sum(ob.y, ta0.y, tb0.y, 0, 0);
+                oa.x = sum(oa.x, ta0.x, tb1.x, ta1.x, tb0.x);
+                oa.y = sum(oa.y, ta0.y, tb1.y, ta1.y, tb0.y);
+            }
         }
         *reinterpret_cast<ulonglong2*>(xb + i) = ob;
         *reinterpret_cast<ulonglong2*>(xa + i) = oa;
@@ -701,7 +729,7 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
 // inverse, pass A: row stages logN-1..LR (GS), with fused prologue
 // ---------------------------------------------------------------------------
 // Prologue modes of the inverse row pass (per segment): IL_PLAIN reads `in`,
-// IL_MUL the product in*in2, IL_AXPY_PINV in + in2*P^-1.
+// IL_MUL the product in*in2.
 template <int LR, int LC, bool FP>
 __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
     k_ntt_inv_rows(const __grid_constant__ DevCtx ctx, const __grid_constant__ LimbMap map) {
@@ -751,17 +779,11 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
             }
         } else {
             const uint64_t* in2 = lr.in2 + base + 2 * lane;
-            const bool mul = lr.lmode == IL_MUL;
             // double-precision limbs: exact products, centred (the schedule's entry bound)
-            const double2 cf = fp && !mul ? *reinterpret_cast<const double2*>(ctx.md_pinvf + 2 * lr.prime) : make_double2(0, 0);
-            const ulonglong2 pi = !fp && !mul ? ldg2(ctx.md_pinv, lr.prime) : make_ulonglong2(0, 0);
             auto one = [&](uint64_t a, uint64_t b) -> uint64_t {
-                if (fp) {
-                    const double x = as_f64(fp_from_u(a)), y = as_f64(fp_from_u(b));
-                    const double r = mul ? fp_mulmod(x, y, p, pinv) : __dadd_rn(x, fp_mulw(y, cf.x, cf.y, p));
-                    return as_u64(fp_center(r, p, pinv));
-                }
-                return mul ? mul_mod(a, b, pc) : add_mod(a, mul_shoup(b, pi.x, pi.y, pc.p), pc.p);
+                if (fp)
+                    return as_u64(fp_center(fp_mulmod(as_f64(fp_from_u(a)), as_f64(fp_from_u(b)), p, pinv), p, pinv));
+                return mul_mod(a, b, pc);
             };
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
@@ -899,6 +921,7 @@ __global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
 // grid (tiles, batch element, limb): CTAs run x fastest, then y, so the
 // elements of a batch that share a prime run together and its twiddle table is
 // fetched from HBM once per launch rather than once per element
+
 template <int LR, int LC>
 struct NttN {
     using CG = ColGeo<LR, LC>;
@@ -930,18 +953,19 @@ struct NttN {
     }
 
     template <bool FP>
-    static void rows_ks_v(const DevCtx& ctx, const KsFuseArgs& a, int nb, cudaStream_t st) {
+    static void rows_ks_v(const DevCtx& ctx, const KsHmultArgs& a, int nb, cudaStream_t st) {
         const int n = a.level + 1, nd = a.level / ctx.alpha + 1;
         auto bytes = [](int tiles) { return ks_warp_words<LR, LC>(tiles) * 8 * RG::W; };
         auto grid = [&](int limbs) { return dim3(RG::GROUPS / RG::W, nb, limbs); };
-        KsFuseArgs q = a;
+        KsHmultArgs q = a;
+        q.nd = nd;
         q.m0 = 0;
         if (ctx.ks_variant & 8) {
             // split launch: the ciphertext-prime outputs need one tile less
-            // (their own digit's value is the input limb) and run at 6 CTAs of
-            // four warps per SM; the special-prime outputs keep every digit's
-            // tile at 4 per SM
-            KsFuseArgs sp = a;
+            // (their own digit's value is a product of input limbs) and run at
+            // 6 CTAs of four warps per SM; the special-prime outputs, with a
+            // tile for every digit, at 4
+            KsHmultArgs sp = q;
             sp.m0 = n;
             count_launches(1);
             launch_pdl(k_ntt_fwd_rows_ks<LR, LC, FP, 6>, grid(n), RG::NT, bytes(nd - 1), st, ctx, q, nd - 1);
@@ -950,7 +974,7 @@ struct NttN {
         }
         launch_pdl(k_ntt_fwd_rows_ks<LR, LC, FP, 4>, grid(n + ctx.K), RG::NT, bytes(nd), st, ctx, q, nd);
     }
-    static void rows_ks(const DevCtx& ctx, const KsFuseArgs& a, int nb, cudaStream_t st) {
+    static void rows_ks(const DevCtx& ctx, const KsHmultArgs& a, int nb, cudaStream_t st) {
         if (ntt_fwd_is_fp(ctx.ntt_variant))
             rows_ks_v<true>(ctx, a, nb, st);
         else
