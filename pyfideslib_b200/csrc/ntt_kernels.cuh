@@ -196,6 +196,14 @@ __device__ __forceinline__ void fp_inv(uint64_t (&x)[16], Get get, double p, dou
 }
 
 // ---- geometry ----
+// Every kernel has two instances: one held to 80 registers, 24 warps per SM, and
+// a wide one of up to 128 registers for launches that do not fill the SMs anyway
+// (kWideThreads): with all the loads of a thread in flight and no spills its
+// warps are shorter, which is all that counts there.
+constexpr int min_ctas(int nt, bool wide) {
+    const int c = (wide ? 512 : 768) / nt;
+    return c < 32 ? c : 32;
+}
 // Column pass: 16 consecutive columns per CTA, TPC threads per column.  (Tiles
 // of 256 threads whatever the column length left a 2^13 transform of 6 limbs
 // on 24 CTAs; 16 columns are the narrowest tile with 128-byte rows.)
@@ -203,7 +211,7 @@ template <int LR, int LC>
 struct ColGeo {
     static constexpr int R = 1 << LR, C = 1 << LC;
     static constexpr int TPC = 1 << (LR - 4), TC = 16, NT = TPC * TC;
-    static constexpr int MINB = 768 / NT < 32 ? 768 / NT : 32;  // 80 registers
+    static constexpr int MINB = min_ctas(NT, false), MINB_WIDE = min_ctas(NT, true);
 };
 // Row pass: a warp (WL lanes, 16 for N = 256) owns RW whole rows = GW
 // contiguous words; W warps per CTA, independent of one another.
@@ -217,7 +225,7 @@ struct RowGeo {
     static constexpr int GROUPS = R * C / GW;
     static constexpr int W = GROUPS < 4 ? GROUPS : 4;
     static constexpr int NT = W * WL;
-    static constexpr int MINB = 768 / NT < 32 ? 768 / NT : 32;
+    static constexpr int MINB = min_ctas(NT, false), MINB_WIDE = min_ctas(NT, true);
     static constexpr unsigned MASK = WL == 32 ? 0xffffffffu : (1u << WL) - 1;
     // staged twiddles of a warp: entry r * 15 + 2^t - 1 + g of row r's first
     // four stages, then psi_br[g], g < 8
@@ -267,8 +275,8 @@ __device__ __forceinline__ ulonglong2 form_tw(const ulonglong2 D, double gw, int
 // ---------------------------------------------------------------------------
 // forward, pass 1: column stages 0..LR-1
 // ---------------------------------------------------------------------------
-template <int LR, int LC, bool FP>
-__global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
+template <int LR, int LC, bool FP, bool WIDE>
+__global__ void __launch_bounds__(ColGeo<LR, LC>::NT, WIDE ? ColGeo<LR, LC>::MINB_WIDE : ColGeo<LR, LC>::MINB)
     k_ntt_fwd_cols(const __grid_constant__ DevCtx ctx, const __grid_constant__ LimbMap map) {
     using G = ColGeo<LR, LC>;
     constexpr int C = G::C, TC = G::TC, LOGN = LR + LC;
@@ -425,8 +433,8 @@ __device__ __forceinline__ void row_epilogue(const LimbRef& lr, size_t base, con
     }
 }
 
-template <int LR, int LC, bool FP>
-__global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
+template <int LR, int LC, bool FP, bool WIDE>
+__global__ void __launch_bounds__(RowGeo<LR, LC>::NT, WIDE ? RowGeo<LR, LC>::MINB_WIDE : RowGeo<LR, LC>::MINB)
     k_ntt_fwd_rows(const __grid_constant__ DevCtx ctx, const __grid_constant__ LimbMap map) {
     using G = RowGeo<LR, LC>;
     __shared__ __align__(16) uint64_t sm[G::W * G::SW];
@@ -730,8 +738,8 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
 // ---------------------------------------------------------------------------
 // Prologue modes of the inverse row pass (per segment): IL_PLAIN reads `in`,
 // IL_MUL the product in*in2.
-template <int LR, int LC, bool FP>
-__global__ void __launch_bounds__(RowGeo<LR, LC>::NT, RowGeo<LR, LC>::MINB)
+template <int LR, int LC, bool FP, bool WIDE>
+__global__ void __launch_bounds__(RowGeo<LR, LC>::NT, WIDE ? RowGeo<LR, LC>::MINB_WIDE : RowGeo<LR, LC>::MINB)
     k_ntt_inv_rows(const __grid_constant__ DevCtx ctx, const __grid_constant__ LimbMap map) {
     using G = RowGeo<LR, LC>;
     constexpr int NST2 = LC - 4;
@@ -847,8 +855,8 @@ __device__ __forceinline__ const uint64_t* inv_scale_entry(const DevCtx& ctx, co
     }
 }
 
-template <int LR, int LC, bool FP>
-__global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
+template <int LR, int LC, bool FP, bool WIDE>
+__global__ void __launch_bounds__(ColGeo<LR, LC>::NT, WIDE ? ColGeo<LR, LC>::MINB_WIDE : ColGeo<LR, LC>::MINB)
     k_ntt_inv_cols(const __grid_constant__ DevCtx ctx, const __grid_constant__ LimbMap map) {
     using G = ColGeo<LR, LC>;
     constexpr int C = G::C, TC = G::TC;
@@ -921,6 +929,11 @@ __global__ void __launch_bounds__(ColGeo<LR, LC>::NT, ColGeo<LR, LC>::MINB)
 // grid (tiles, batch element, limb): CTAs run x fastest, then y, so the
 // elements of a batch that share a prime run together and its twiddle table is
 // fetched from HBM once per launch rather than once per element
+// Threads up to which a launch takes the wide instances: what the narrow ones
+// hold in one wave.  N = 2^16, 50-bit limbs, narrow / wide: 18 limbs 15.0 / 11.2 us
+// forward, 24 limbs 14.8 / 15.3, 29 limbs 17.0 / 18.2; N = 2^15, 59-bit limbs, 2 x 20
+// limbs 25.1 / 22.2, 2 x 29 limbs 28.7 / 29.1.
+constexpr size_t kWideThreads = (size_t)768 * 148;
 
 template <int LR, int LC>
 struct NttN {
@@ -929,26 +942,30 @@ struct NttN {
     static dim3 gcols(const LimbMap& m) { return dim3(CG::C / CG::TC, m.nb > 0 ? m.nb : 1, m.total); }
     static dim3 grows(const LimbMap& m) { return dim3(RG::GROUPS / RG::W, m.nb > 0 ? m.nb : 1, m.total); }
 
+    template <class K>
+    static void launch(K narrow, K wide, dim3 g, int nt, const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
+        launch_pdl((size_t)g.x * g.y * g.z * nt <= kWideThreads ? wide : narrow, g, nt, 0, st, ctx, map);
+    }
     static void fwd_cols(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
         if (ntt_fwd_is_fp(ctx.ntt_variant))
-            launch_pdl(k_ntt_fwd_cols<LR, LC, true>, gcols(map), CG::NT, 0, st, ctx, map);
+            launch(k_ntt_fwd_cols<LR, LC, true, false>, k_ntt_fwd_cols<LR, LC, true, true>, gcols(map), CG::NT, ctx, map, st);
         else
-            launch_pdl(k_ntt_fwd_cols<LR, LC, false>, gcols(map), CG::NT, 0, st, ctx, map);
+            launch(k_ntt_fwd_cols<LR, LC, false, false>, k_ntt_fwd_cols<LR, LC, false, true>, gcols(map), CG::NT, ctx, map, st);
     }
     static void fwd(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
         fwd_cols(ctx, map, st);
         if (ntt_fwd_is_fp(ctx.ntt_variant))
-            launch_pdl(k_ntt_fwd_rows<LR, LC, true>, grows(map), RG::NT, 0, st, ctx, map);
+            launch(k_ntt_fwd_rows<LR, LC, true, false>, k_ntt_fwd_rows<LR, LC, true, true>, grows(map), RG::NT, ctx, map, st);
         else
-            launch_pdl(k_ntt_fwd_rows<LR, LC, false>, grows(map), RG::NT, 0, st, ctx, map);
+            launch(k_ntt_fwd_rows<LR, LC, false, false>, k_ntt_fwd_rows<LR, LC, false, true>, grows(map), RG::NT, ctx, map, st);
     }
     static void inv(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
         if (ntt_inv_is_fp(ctx.intt_variant)) {
-            launch_pdl(k_ntt_inv_rows<LR, LC, true>, grows(map), RG::NT, 0, st, ctx, map);
-            launch_pdl(k_ntt_inv_cols<LR, LC, true>, gcols(map), CG::NT, 0, st, ctx, map);
+            launch(k_ntt_inv_rows<LR, LC, true, false>, k_ntt_inv_rows<LR, LC, true, true>, grows(map), RG::NT, ctx, map, st);
+            launch(k_ntt_inv_cols<LR, LC, true, false>, k_ntt_inv_cols<LR, LC, true, true>, gcols(map), CG::NT, ctx, map, st);
         } else {
-            launch_pdl(k_ntt_inv_rows<LR, LC, false>, grows(map), RG::NT, 0, st, ctx, map);
-            launch_pdl(k_ntt_inv_cols<LR, LC, false>, gcols(map), CG::NT, 0, st, ctx, map);
+            launch(k_ntt_inv_rows<LR, LC, false, false>, k_ntt_inv_rows<LR, LC, false, true>, grows(map), RG::NT, ctx, map, st);
+            launch(k_ntt_inv_cols<LR, LC, false, false>, k_ntt_inv_cols<LR, LC, false, true>, gcols(map), CG::NT, ctx, map, st);
         }
     }
 
