@@ -43,13 +43,13 @@ LOGN, L, K, DNUM = 16, 30, 10, 3
 # DRAM bytes (read + write) of one batched forward NTT (32 polynomials x 30
 # limbs at N=2^16): a constant taken from one ncu capture of that launch pair
 # (dram__bytes_read.sum + dram__bytes_write.sum of k_ntt_fwd_cols and
-# k_ntt_fwd_rows, forward variant 9, caches flushed before each kernel), stale
+# k_ntt_fwd_rows, FP64 butterflies, caches flushed before each kernel), stale
 # after any change to those kernels; --ntt-traffic-csv reads a fresh capture
 # instead.  About twice the algorithmic bytes: the column pass writes the 960
 # intermediate limbs (480 MB, more than L2) and the row pass reads them back;
 # twiddles add 32 MB (read once per prime for the whole batch).
-NTT_BATCH_TRAFFIC_BYTES = 1922.8e6  # 503.5 + 443.3 (cols) + 535.0 + 441.0 (rows) MB
-NTT_BATCH_TRAFFIC_SOURCE = "constant from one ncu capture of the launch pair (variant 9, caches flushed)"
+NTT_BATCH_TRAFFIC_BYTES = 1924.1e6  # 503.5 + 445.4 (cols) + 534.7 + 440.5 (rows) MB
+NTT_BATCH_TRAFFIC_SOURCE = "constant from one ncu capture of the launch pair (FP64 butterflies, caches flushed)"
 _UNITS = {"byte": 1.0, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9, "Tbyte": 1e12}
 
 

@@ -88,11 +88,11 @@ const char* fides_ctx_last_error(const fides_ctx* ctx);
  * callers that time or order work around it (FIDESlib keeps per-partition
  * streams in ContextData, src/CKKS/Context.cuh:85-98). */
 fides_status fides_ctx_stream(const fides_ctx* ctx, void** stream);
-/* Autotuner: time every forward NTT variant (occupancy, twiddle-fetch
- * policy, integer or double-precision butterflies, row twiddles staged or
- * formed in the kernel) and every inverse configuration on one element's
- * ModUp digits and on the same shape batched over four elements, and keep
- * the fastest of each (sum of the two times).
+/* Autotuner: time the forward and inverse NTT with integer butterflies on
+ * every limb (forward variants 0-4, inverse configurations 0-2) and with
+ * double-precision ones on the limbs of primes below 2^50 (5-9, 3-5) on one
+ * element's ModUp digits and on the same shape batched over four elements,
+ * and keep the fastest of each (sum of the two times).
  * Runs once in fides_ctx_create; call again to re-tune.  *variant receives
  * the forward variant, times_ms[v] (num_variants entries, at most 16) the
  * forward time of variant v plus that of its paired inverse configuration;

@@ -48,7 +48,7 @@ __device__ __forceinline__ uint64_t uniform_mod(uint64_t stream, int prime, uint
 struct DevCtx {
     int logN, N, L, K, dnum, alpha;
     int ntt_variant;             // forward NTT kernel variant chosen by the autotuner
-    int intt_variant;            // inverse NTT kernel configuration (0..2)
+    int intt_variant;            // inverse NTT kernel configuration (ntt.cu)
     int ks_variant;              // key-switch inner product: bit 0 set: FP64 sums on primes below 2^50
                                  // (else integer sums); bit 1 set: HMult's inner product runs in the
                                  // epilogue of the ModUp digits' NTT row pass (else its own kernel);
