@@ -111,6 +111,8 @@ struct LimbSeg {
     size_t bstride;  // batch element b adds b * bstride words to in/in2/out
 };
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 struct LimbMap {
     int nseg;
     int total;

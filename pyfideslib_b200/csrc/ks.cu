@@ -408,14 +408,15 @@ void launch_ks_inner(const DevCtx& ctx, int level, int nb, const KsArgs& args, c
 //   XA[m] = a0 b1 + a1 b0 + P^-1 sum_d D_d[t] ka[d][t]      (m < n),
 // the special limbs as the sums.  Bounds and sums as in k_ks_inner.
 // ---------------------------------------------------------------------------
-// HBM bounds this kernel in a batch, its loads' latency in a single product.
+// Its loads' latency bounds this kernel (8 pairs: 8 of 16 stall cycles per
+// instruction, DRAM 53%).
 // ModUp's inverse transform takes a1 b1 in its own load, so no limb of the
 // tensor product is stored: 8 limbs of traffic per limb of the level instead of
 // 13 around the tensor product, that inverse, this kernel and the final row
 // pass, and one launch less.  64 registers: 4 CTAs per SM, without spills (left
 // free it takes 72, 3 CTAs, one product at N = 2^16 258 us instead of 251).
-// N = 2^16, L = 30, with a tensor kernel / this: one product 260 / 251 us, 21
-// pairs at uneven levels 6449 / 6122 us.  Large batches form these sums in the
+// N = 2^16, L = 30, with a tensor kernel / this: one product 260 / 248 us, 21
+// pairs at uneven levels 6449 / 6072 us.  Large batches form these sums in the
 // epilogue of the digits' row pass instead (k_ntt_fwd_rows_ks).
 template <bool FPK, bool SEED>
 __global__ void __launch_bounds__(256, 4)
@@ -434,11 +435,11 @@ __global__ void __launch_bounds__(256, 4)
     const size_t koff = (size_t)t * ctx.N + j;
     auto word = [&](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q + koff); };
     auto own_digit = [&](int d) { return tensor && (unsigned)(m - d * ctx.alpha) < (unsigned)ctx.alpha; };
-    auto digit = [&](int d) {  // ModUp output of digit d: the Q primes outside it, then the special primes
+    auto digit_at = [&](int d) {  // ModUp output of digit d: the Q primes outside it, then the special primes
         const int lo = d * ctx.alpha, cnt = min(ctx.alpha, n - lo);
-        return *reinterpret_cast<const ulonglong2*>(
-            args.dig + boff + ((size_t)d * args.dig_stride + (m < lo ? m : m - cnt)) * ctx.N + j);
+        return args.dig + boff + ((size_t)d * args.dig_stride + (m < lo ? m : m - cnt)) * ctx.N + j;
     };
+    auto digit = [&](int d) { return *reinterpret_cast<const ulonglong2*>(digit_at(d)); };
     auto key_a = [&](int d) {
         ulonglong2 a;
         if (!SEED) {
@@ -449,6 +450,15 @@ __global__ void __launch_bounds__(256, 4)
         }
         return a;
     };
+    // The later digits' words are asked for at the start: left to the loop, each
+    // digit waited for HBM in turn (one product at N = 2^16, L = 30 251 us instead of
+    // 248, 21 pairs 6094 instead of 6072).  In k_ks_inner, whose digits come from
+    // L2, the same for its keys was 0.3-1% slower.
+    for (int d = 1; d < nd; ++d) {
+        prefetch_l2(args.kb + d * kstride + koff);
+        if (!SEED) prefetch_l2(args.ka + d * kstride + koff);
+        if (!own_digit(d)) prefetch_l2(digit_at(d));
+    }
     ulonglong2 a0, a1, b0, b1;
     if (tensor) {
         a0 = word(args.a0[bi]);

@@ -114,7 +114,6 @@ __device__ __forceinline__ void gs_bfly_fp(uint64_t& X, uint64_t& Y, const ulong
     Y = as_u64(fp_mulw(__dsub_rn(x, y), as_f64(w.x), as_f64(w.y), p));
 }
 
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ ulonglong2 ldg2(const uint64_t* base, size_t idx) {
     return __ldg(reinterpret_cast<const ulonglong2*>(base) + idx);
