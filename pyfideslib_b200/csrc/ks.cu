@@ -1,5 +1,5 @@
-// ks.cu -- tensor product, ModUp / ModDown base conversions, the hybrid
-// key-switch inner product and the element-wise kernels, for sm_100a.
+// ks.cu -- ModUp / ModDown base conversions, the hybrid key-switch inner
+// products (with the tensor product) and the element-wise kernels, for sm_100a.
 //
 // Role in the reference: src/CKKS/Conv.cu (DecompAndModUpConv, ModDown2),
 // src/CKKS/ElemenwiseBatchKernels.cu (binomialMult_, fusedDotKSK_2_,
@@ -230,11 +230,11 @@ void launch_modup_conv(const DevCtx& ctx, int level, int nb, const uint64_t* xt,
 // stays below 7p < 2^53, and one centring plus a floor reduction give the
 // canonical residue -- the same values as the 128-bit integer sums.
 // SEED: some element's key is seeded (ka null), its a half regenerated per
-// coefficient; the instantiation without it carries no generator code and
-// keeps the register count of the plain streaming loop (32-40).  Left free,
-// the unrolled digit loop with the generator takes 56-72 registers; the
-// bound holds it at 48 (FP64 sums) or 40 so that 5-6 blocks stay resident
-// (not the split-product accumulator, which would spill).
+// coefficient; the instantiation without it carries no generator code (52
+// registers; 48 measured the same).  Left free, the unrolled digit loop with
+// the generator takes 56-72; the bound holds it at 48 (FP64 sums) or 40 so that
+// 5-6 blocks stay resident (not the split-product accumulator, which would
+// spill).
 template <class ACC>
 constexpr bool kIsSplitAcc = false;
 template <>
