@@ -411,17 +411,22 @@ fides_status fides_srv_destroy(fides_server* srv);
 
 /* ---- raw limb kernels on device memory (LimbPartition NTT/INTT entry points,
  *      src/CKKS/LimbPartition.cu; used for the plain RNS polynomial multiply) ---- */
-/* In-place forward / inverse NTT of `nlimbs` limbs at `data` (device pointer),
- * limb i using prime index prime0 + i. */
+/* In-place forward / inverse NTT of `nlimbs` limbs of canonical residues at
+ * `data` (device pointer), limb i using prime index prime0 + i.  A forward
+ * transform needs data on a 16-byte boundary (FIDES_BAD_ARG otherwise), an
+ * inverse one on an 8-byte boundary. */
 fides_status fides_ntt(fides_ctx* ctx, uint64_t* data, int prime0, int nlimbs, int inverse);
 /* The same transform over npoly polynomials of nlimbs limbs each, polynomial k
  * at data + k * poly_stride words, in one launch pair (the batched form the
- * key-switch pipeline uses; LimbPartitionBatch.cu runs NTT_ per partition). */
+ * key-switch pipeline uses; LimbPartitionBatch.cu runs NTT_ per partition).
+ * The boundaries of fides_ntt hold for every polynomial: forward, poly_stride
+ * is even. */
 fides_status fides_ntt_batch(fides_ctx* ctx, uint64_t* data, size_t poly_stride, int npoly, int prime0, int nlimbs,
                              int inverse);
 /* c = a * b in R_q for nlimbs limbs of coefficient-form inputs (device
  * pointers): NTT of a and b into a_ntt / b_ntt (caller-provided device
- * scratch), then one INTT with the product fused into its load.  `c` may
+ * scratch on 16-byte boundaries, FIDES_BAD_ARG otherwise; a, b and c on 8-byte
+ * ones), then one INTT with the product fused into its load.  `c` may
  * alias a or b. */
 fides_status fides_polymul(fides_ctx* ctx, const uint64_t* a, const uint64_t* b, uint64_t* c, uint64_t* a_ntt,
                            uint64_t* b_ntt, int prime0, int nlimbs);

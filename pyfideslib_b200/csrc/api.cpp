@@ -1674,10 +1674,15 @@ fides_status fides_plan_free(fides_ctx* c, fides_plan* plan) {
     return FIDES_OK;
 }
 
+// the forward row pass stores 16-byte words
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 fides_status fides_ntt(fides_ctx* ctx, uint64_t* data, int prime0, int nlimbs, int inverse) {
     if (!ctx || !data || prime0 < 0 || nlimbs < 1 || prime0 + nlimbs > ctx->L + ctx->K || nlimbs > 65535)
         return FIDES_BAD_ARG;
     Guard g(ctx);
+    if (!inverse && !aligned16(data))
+        return set_err(ctx, FIDES_BAD_ARG, "forward transform: data must start on a 16-byte boundary");
     LimbMap m = map_single(data, data, nlimbs, nlimbs, prime0);
     if (inverse)
         ntt_inverse(ctx->dev, m, IL_PLAIN, IS_PLAIN, ctx->st);
@@ -1692,6 +1697,8 @@ fides_status fides_ntt_batch(fides_ctx* ctx, uint64_t* data, size_t poly_stride,
         prime0 + nlimbs > ctx->L + ctx->K || poly_stride < (size_t)nlimbs * ctx->N)
         return FIDES_BAD_ARG;
     Guard g(ctx);
+    if (!inverse && (!aligned16(data) || (npoly > 1 && (poly_stride & 1))))
+        return set_err(ctx, FIDES_BAD_ARG, "forward transform: every polynomial must start on a 16-byte boundary");
     LimbMap m = map_single(data, data, nlimbs, nlimbs, prime0);
     m.nb = npoly;
     m.seg[0].bstride = poly_stride;
@@ -1708,6 +1715,8 @@ fides_status fides_polymul(fides_ctx* ctx, const uint64_t* a, const uint64_t* b,
         prime0 + nlimbs > ctx->L + ctx->K || nlimbs > 32767)
         return FIDES_BAD_ARG;
     Guard g(ctx);
+    if (!aligned16(a_ntt) || !aligned16(b_ntt))
+        return set_err(ctx, FIDES_BAD_ARG, "polymul: a_ntt and b_ntt must start on a 16-byte boundary");
     LimbMap m{};
     m.nseg = 2;
     const uint64_t* ins[2] = {a, b};

@@ -769,7 +769,15 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, WIDE ? RowGeo<LR, LC>::MIN
     const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
     pdl_wait();
     uint64_t x[16];
-    {
+    if (reinterpret_cast<uintptr_t>(lr.in) & 15) {
+        // a caller's limbs may start at an odd word (fides_ntt, fides_ntt_batch
+        // with an odd stride; always IL_PLAIN): 8-byte loads, one by one
+#pragma unroll 1
+        for (int i = lane; i < G::GW; i += G::WL) {
+            const uint64_t u = lr.in[base + i];
+            sw[padi(i)] = fp ? fp_from_u(u) : u;
+        }
+    } else {
         // all 16 words of the lane are loaded before any is used, so the
         // global loads (twice as many with a second operand) are in flight together
         ulonglong2 v[8];
