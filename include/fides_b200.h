@@ -272,8 +272,12 @@ fides_status fides_rotate_batch(fides_ctx* ctx, int n, const fides_ct* const* a,
  * output and intermediate buffer and captures the kernel sequence once;
  * fides_plan_launch replays it (a single graph launch) on the context
  * stream, reading the inputs' current residues (fides_ct_write refreshes
- * them).  a, b and out must outlive the plan.  No counterpart in the
- * reference, which captures per-level graphs of one key switch
+ * them).  a, b and out must outlive the plan and keep their buffers: once
+ * another operation has written its result into one of them (or a key was
+ * stored in another form, or a compressed one generated from another seed), the
+ * launch returns FIDES_BAD_ARG and the plan has to be made again.  The plan
+ * keeps the workspace it was captured with.  No counterpart in the reference,
+ * which captures per-level graphs of one key switch
  * (LimbPartitionMGPU.cu:581-640, FIDESLIB_USE_GRAPH_CAPTURE). */
 fides_status fides_plan_hmult_rotate(fides_ctx* ctx, int n, const fides_ct* const* a, const fides_ct* const* b,
                                      const int32_t* indices, int rescale, fides_ct* const* out, fides_plan** plan);

@@ -1524,6 +1524,20 @@ struct fides_plan {
     cudaGraphExec_t exec = nullptr;
     std::vector<fides_ct> inter;  // products feeding the rotations
     std::vector<fides_ct*> outs;  // written by every replay
+    // what the graph's kernels point at: the batch workspace (kept alive), the
+    // ciphertexts' buffers and the keys (checked before every replay)
+    std::shared_ptr<WsMem> ws;
+    struct CtRef {
+        const fides_ct* ct;
+        const uint64_t* buf;
+        int cap;
+    };
+    struct KeyRef {
+        const SwitchKey* key;
+        SwitchKey was;
+    };
+    std::vector<CtRef> cts;
+    std::vector<KeyRef> keys;
 };
 
 extern "C" {
@@ -1636,6 +1650,16 @@ fides_status fides_plan_hmult_rotate(fides_ctx* c, int n, const fides_ct* const*
     }
     p->graph = graph;
     p->nkernels = launch_count() - k0count;
+    p->ws = c->wsb.mem;
+    auto& refs = c->plan_ws;
+    refs.erase(std::remove_if(refs.begin(), refs.end(), [](const std::weak_ptr<WsMem>& m) { return m.expired(); }),
+               refs.end());
+    refs.push_back(p->ws);
+    p->keys.push_back({&c->relin, c->relin});
+    for (int i = 0; i < n; ++i) {
+        for (const fides_ct* t : {a[i], b[i], (const fides_ct*)out[i]}) p->cts.push_back({t, t->buf, t->cap});
+        if (keys[i]) p->keys.push_back({keys[i], *keys[i]});
+    }
     const cudaError_t e2 = cudaGraphInstantiate(&p->exec, graph, 0);
     if (e2 != cudaSuccess) {
         fides_plan_free(c, p);
@@ -1656,6 +1680,12 @@ fides_status fides_plan_hmult_rotate(fides_ctx* c, int n, const fides_ct* const*
 fides_status fides_plan_launch(fides_ctx* c, fides_plan* plan) {
     if (!c || !plan || !plan->exec) return FIDES_BAD_ARG;
     Guard g(c);
+    for (const auto& r : plan->cts)
+        if (r.ct->buf != r.buf || r.ct->cap != r.cap)
+            return set_err(c, FIDES_BAD_ARG, "plan: an operation replaced the buffer of one of its ciphertexts");
+    for (const auto& r : plan->keys)
+        if (r.key->b != r.was.b || r.key->a != r.was.a || (!r.was.a && r.key->a_seed != r.was.a_seed))
+            return set_err(c, FIDES_BAD_ARG, "plan: one of its switching keys was replaced");
     for (fides_ct* o : plan->outs) ct_quiesce(c, o);  // pending downloads of the last replay's results
     count_launches((int)plan->nkernels);
     if (cudaGraphLaunch(plan->exec, c->st) != cudaSuccess) return check_cuda(c, "graph launch");

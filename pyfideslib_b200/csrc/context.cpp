@@ -583,11 +583,13 @@ fides_status ws_reserve(fides_ctx* c, Workspace& w, int cap) {
     const size_t limbs = L /*XT*/ + c->dnum * w.dig_stride /*DIG*/ + 2 * (L + K) /*XB,XA*/ +
                          2 * L /*W*/ + 2 /*T*/;
     w.stride = limbs * N;
-    if (cudaMalloc((void**)&w.base, w.stride * 8 * (size_t)cap) != cudaSuccess) {
+    w.mem = std::make_shared<WsMem>();
+    if (cudaMalloc((void**)&w.mem->p, w.stride * 8 * (size_t)cap) != cudaSuccess) {
         cudaGetLastError();
-        w.base = nullptr;
+        w.mem->p = nullptr;
         return set_err(c, FIDES_OOM, "workspace allocation failed");
     }
+    w.base = w.mem->p;
     w.cap = cap;
     uint64_t* p = w.base;
     auto take = [&](size_t n) {
@@ -604,10 +606,11 @@ fides_status ws_reserve(fides_ctx* c, Workspace& w, int cap) {
     return FIDES_OK;
 }
 
-void ws_free(Workspace& w) {
-    if (w.base) cudaFree(w.base);
-    w = Workspace{};
+WsMem::~WsMem() {
+    if (p) cudaFree(p);
 }
+
+void ws_free(Workspace& w) { w = Workspace{}; }
 
 void free_context(fides_ctx* c) {
     if (!c) return;
@@ -624,6 +627,12 @@ void free_context(fides_ctx* c) {
     c->galois_keys.clear();
     ws_free(c->ws1);
     ws_free(c->wsb);
+    for (auto& m : c->plan_ws)
+        if (auto ws = m.lock()) {
+            if (ws->p) cudaFree(ws->p);
+            ws->p = nullptr;
+        }
+    c->plan_ws.clear();
     if (c->table_mem) cudaFree(c->table_mem);
     if (c->tc_mem) cudaFree(c->tc_mem);
     c->tc_mem = nullptr;

@@ -59,9 +59,16 @@ struct SwitchKey {
 
 // Key-switch workspace for `cap` batch elements; element b's buffers sit at
 // the element-0 pointers + b*stride words.  Sized for the top level.
+struct WsMem {
+    uint64_t* p = nullptr;
+    ~WsMem();
+};
 struct Workspace {
     cudaStream_t st = nullptr;  // stream the engine queues this workspace's work on
     uint64_t* base = nullptr;
+    // base's owner: a captured plan shares it, so that a larger batch, which
+    // takes a new allocation, leaves the one its graph works in alive
+    std::shared_ptr<WsMem> mem;
     size_t stride = 0;  // words per element
     int cap = 0;
     size_t dig_stride = 0;  // limbs per digit in DIG
@@ -104,6 +111,7 @@ struct fides_ctx {
     // (allocated on first use) for batches
     fides::Workspace ws1;
     fides::Workspace wsb;
+    std::vector<std::weak_ptr<fides::WsMem>> plan_ws;  // workspaces that plans share, freed with the context
 
     fides::SwitchKey relin;
     bool has_relin = false;
