@@ -525,7 +525,7 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
     d.md_pinvf = (const double*)(base + parts[i_dpf].off);
     d.rs_qinvf = (const double*)(base + parts[i_rqf].off);
     d.err = (uint32_t*)(base + parts[i_err].off);
-    ntt_prepare(d);
+    if (ntt_prepare(d) != cudaSuccess) return set_err(c, FIDES_CUDA_ERR, "shared-memory opt-in of the transforms failed");
     d.tc_btab = nullptr;
     d.tc_boff = nullptr;
     if (conv_tc_eligible(d)) {

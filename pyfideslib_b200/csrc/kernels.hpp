@@ -57,7 +57,7 @@ struct NttOps {
     void (*inv)(const DevCtx&, const LimbMap&, cudaStream_t);
     void (*fwd_cols)(const DevCtx&, const LimbMap&, cudaStream_t);
     void (*rows_ks)(const DevCtx&, const KsHmultArgs&, int nb, cudaStream_t);
-    void (*prepare)(const DevCtx&);
+    cudaError_t (*prepare)();
 };
 template <int LOGN>
 const NttOps& ntt_ops();
@@ -75,7 +75,7 @@ int ntt_inverse_of(int forward_variant);
 void ntt_forward(const DevCtx& ctx, const LimbMap& map, int load, int store, cudaStream_t st);
 // Per-device set-up of this ring dimension's kernels (the fused kernel's
 // shared-memory opt-in), before any launch or stream capture.
-void ntt_prepare(const DevCtx& ctx);
+cudaError_t ntt_prepare(const DevCtx& ctx);
 // Forward NTT column pass alone (seg.in -> seg.out), for the fused key switch.
 void ntt_forward_cols(const DevCtx& ctx, const LimbMap& map, int load, cudaStream_t st);
 // HMult's inner product with the rest of its tensor product, for nb batch
@@ -104,7 +104,9 @@ struct KsHmultArgs {
 };
 // its form fused into the digits' row pass (DIG after the column pass)
 void ntt_rows_keyswitch(const DevCtx& ctx, const KsHmultArgs& a, int nb, cudaStream_t st);
-// the fused row pass keeps one transformed tile per digit in shared memory
+// the fused row pass keeps one transformed tile per digit in shared memory, and
+// its epilogue's sums take at most six digits
+constexpr int kMaxFusedDigits = 6;
 bool ntt_rows_keyswitch_supported(const DevCtx& ctx);
 // Inverse NTT: pass A reads seg.in (+in2 for the prologue), writes seg.out;
 // pass B finishes seg.out in place.

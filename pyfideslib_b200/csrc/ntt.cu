@@ -67,7 +67,7 @@ void ntt_forward(const DevCtx& ctx, const LimbMap& m, int load, int store, cudaS
     ops_of(ctx.logN)->fwd(ctx, map, st);
 }
 
-void ntt_prepare(const DevCtx& ctx) { ops_of(ctx.logN)->prepare(ctx); }
+cudaError_t ntt_prepare(const DevCtx& ctx) { return ops_of(ctx.logN)->prepare(); }
 
 void ntt_forward_cols(const DevCtx& ctx, const LimbMap& m, int load, cudaStream_t st) {
     if (m.total <= 0) return;
@@ -82,8 +82,7 @@ void ntt_rows_keyswitch(const DevCtx& ctx, const KsHmultArgs& a, int nb, cudaStr
     ops_of(ctx.logN)->rows_ks(ctx, a, nb, st);
 }
 
-// one transformed tile per digit and the epilogue's sums of at most six digits
-bool ntt_rows_keyswitch_supported(const DevCtx& ctx) { return ctx.dnum <= 6; }
+bool ntt_rows_keyswitch_supported(const DevCtx& ctx) { return ctx.dnum <= kMaxFusedDigits; }
 
 void ntt_inverse(const DevCtx& ctx, const LimbMap& m, int load, int store, cudaStream_t st) {
     if (m.total <= 0) return;

@@ -1004,13 +1004,20 @@ struct NttN {
         else
             rows_ks_v<false>(ctx, a, nb, st);
     }
-    // shared-memory opt-in of the fused kernel
-    static void prepare(const DevCtx& ctx) {
-        const int bytes = (int)(ks_warp_words<LR, LC>(ctx.dnum) * 8 * RG::W);
-        cudaFuncSetAttribute(k_ntt_fwd_rows_ks<LR, LC, true, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(k_ntt_fwd_rows_ks<LR, LC, true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(k_ntt_fwd_rows_ks<LR, LC, false, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        cudaFuncSetAttribute(k_ntt_fwd_rows_ks<LR, LC, false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    // Shared-memory opt-in of the fused kernel.  The limit belongs to the process
+    // and device, not to a context: it is the most that any context can ask for.
+    static cudaError_t prepare() {
+        const int bytes = (int)(ks_warp_words<LR, LC>(kMaxFusedDigits) * 8 * RG::W);
+        cudaError_t e = cudaSuccess;
+        auto opt_in = [&](auto k) {
+            const cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            if (e == cudaSuccess) e = r;
+        };
+        opt_in(k_ntt_fwd_rows_ks<LR, LC, true, 6>);
+        opt_in(k_ntt_fwd_rows_ks<LR, LC, true, 4>);
+        opt_in(k_ntt_fwd_rows_ks<LR, LC, false, 6>);
+        opt_in(k_ntt_fwd_rows_ks<LR, LC, false, 4>);
+        return e;
     }
 };
 
