@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(256, SEED ? (FPK ? 5 : (kIsSplitAcc<ACC> ? 0 :
         // branch took 851 us for 32 rotations of 20 limbs at N = 2^16, 70% of
         // the issue slots busy.)
         const size_t j = ((size_t)bx * blockDim.x + threadIdx.x) * 2;
+        if (j >= (size_t)ctx.N) return;  // N = 256: half a block
         const uint32_t g = args.galois[bi];
         const uint32_t s0 = g ? automorph_slot(ctx.logN, g, (uint32_t)j) : (uint32_t)j;
         const bool swap = s0 & 1;
@@ -384,7 +385,7 @@ void launch_ks_inner(const DevCtx& ctx, int level, int nb, const KsArgs& args, c
     bool seeded = false;
     for (int b = 0; b < nb; ++b) seeded = seeded || args.ka[b] == nullptr;
     const int nd = level / ctx.alpha + 1;
-    const dim3 g(ctx.N / 512, nb, level + 1 + ctx.K);
+    const dim3 g((ctx.N + 511) / 512, nb, level + 1 + ctx.K);
     if (args.dig_group > 0) {
         if (ctx.ks_variant & 1)
             ks_inner_go<Acc128, true, true>(ctx, level, nd, args, seeded, g, st);
@@ -432,6 +433,7 @@ __global__ void __launch_bounds__(256, 4)
     const size_t kstride = (size_t)(ctx.L + ctx.K) * ctx.N;
     const size_t boff = (size_t)bi * args.bstride;
     const size_t j = ((size_t)blockIdx.x * 256 + threadIdx.x) * 2;
+    if (j >= (size_t)ctx.N) return;  // N = 256: half a block
     const size_t koff = (size_t)t * ctx.N + j;
     auto word = [&](const uint64_t* q) { return *reinterpret_cast<const ulonglong2*>(q + koff); };
     auto own_digit = [&](int d) { return tensor && (unsigned)(m - d * ctx.alpha) < (unsigned)ctx.alpha; };
@@ -544,7 +546,7 @@ __global__ void __launch_bounds__(256, 4)
 
 template <bool FPK>
 static void ks_hmult_go(const DevCtx& ctx, int nb, const KsHmultArgs& args, cudaStream_t st) {
-    const dim3 g(ctx.N / 512, nb, args.level + 1 + ctx.K);
+    const dim3 g((ctx.N + 511) / 512, nb, args.level + 1 + ctx.K);
     if (args.ka == nullptr)
         launch_pdl(k_ks_hmult<FPK, true>, g, 256, 0, st, ctx, args);
     else
