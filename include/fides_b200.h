@@ -108,7 +108,7 @@ fides_status fides_autotune_conv_info(const fides_ctx* ctx, int* accumulator, fl
 /* Force the conversion variant (0..4, for measurements and tests; 3 and 4
  * run the ModUp conversion on the tensor cores as an exact int8-split
  * contraction with 32 or 16 targets per matrix product, digits of at most 16
- * moduli); -1 restores the tuned choice. */
+ * moduli, every modulus above 2^17); -1 restores the tuned choice. */
 fides_status fides_set_conv_accumulator(fides_ctx* ctx, int accumulator);
 /* Key-switch inner product (identical results in every form; for
  * measurements and tests).  Bit 0: the digit products of primes below 2^50

@@ -286,7 +286,8 @@ fides_status fides_set_conv_accumulator(fides_ctx* c, int accumulator) {
         for (uint64_t q : c->host.prime)
             if (q >= (1ull << 60)) return set_err(c, FIDES_UNSUPPORTED, "split products need moduli below 2^60");
     if (accumulator >= 3 && !conv_tc_supported(c->dev))
-        return set_err(c, FIDES_UNSUPPORTED, "tensor-core conversion needs digits of at most 16 moduli and at most 48 targets");
+        return set_err(c, FIDES_UNSUPPORTED,
+                       "tensor-core conversion needs digits of at most 16 moduli, at most 48 targets and moduli above 2^17");
     c->dev.conv_variant = accumulator < 0 ? c->tuned_conv : accumulator;
     return FIDES_OK;
 }

@@ -528,7 +528,7 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
     if (ntt_prepare(d) != cudaSuccess) return set_err(c, FIDES_CUDA_ERR, "shared-memory opt-in of the transforms failed");
     d.tc_btab = nullptr;
     d.tc_boff = nullptr;
-    if (conv_tc_eligible(d)) {
+    if (conv_tc_eligible(d, *std::min_element(c->host.prime.begin(), c->host.prime.end()))) {
         // byte matrices of the tensor-core conversions, one per (level, digit)
         // and per (level, fused) ModDown (a few MB); without them the
         // conversions run on the integer pipes

@@ -47,6 +47,9 @@ constexpr int kTcRows = 128;        // coefficients per tile (MMA M)
 constexpr int kTcCols = 8;          // accumulator columns per target (byte positions 0..7 of V')
 constexpr uint32_t kTcLboA = (kTcRows / 8) * 128;  // A: K-chunk stride in bytes
 constexpr uint32_t kSpinLimit = 1u << 20;
+// smallest modulus of reduce_cols: below it the quotient can be short by two
+// (and below 2^16 its constant no longer fits 32 bits)
+constexpr uint64_t kTcMinModulus = 1ull << 17;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -107,7 +110,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&c)[32]) {
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
-// V' mod p for V' = sum_{s<8} c_s 2^{8s}, c_s < 2^23, 2^17 <= p < 2^62.
+// V' mod p for V' = sum_{s<8} c_s 2^{8s}, c_s < 2^23, 2^17 <= p < 2^62 (kTcMinModulus).
 // The pairs w_k = c_{2k} + c_{2k+1} 2^8 fit 32 bits, and with
 // e = w_0 + w_2 2^32, o = w_1 + w_3 2^32:  V' = e + o 2^16,
 // floor(V'/2^16) = floor(e/2^16) + o  and  V' mod 2^64 = e + (o << 16).
@@ -545,15 +548,15 @@ void launch_tc(const DevCtx& ctx, int level, int groups, int items, int ck, int 
 
 }  // namespace
 
-bool conv_tc_eligible(const DevCtx& ctx) {
-    if (ctx.alpha > 16 || ctx.K > 16) return false;
+bool conv_tc_eligible(const DevCtx& ctx, uint64_t smallest) {
+    if (ctx.alpha > 16 || ctx.K > 16 || smallest < kTcMinModulus) return false;
     const int up = ctx.L - 1 + ctx.K;  // ModUp: at most L-1 other Q primes plus K
     return up <= kTcMaxTargets && ctx.L <= kTcMaxTargets &&
            tc_smem_bytes((ctx.alpha + 3) / 4, up, false) <= kTcSmemCap &&
            tc_smem_bytes((ctx.K + 3) / 4, ctx.L, true) <= kTcSmemCap;
 }
 
-bool conv_tc_supported(const DevCtx& ctx) { return ctx.tc_btab != nullptr && conv_tc_eligible(ctx); }
+bool conv_tc_supported(const DevCtx& ctx) { return ctx.tc_btab != nullptr; }
 
 size_t conv_tc_table_layout(const DevCtx& ctx, std::vector<uint64_t>& offs) {
     const int L = ctx.L, K = ctx.K, dn = ctx.dnum;

@@ -148,8 +148,8 @@ bool conv_supported(const DevCtx& ctx);
 constexpr int kConvVariants = 5;  // see DevCtx::conv_variant
 // ModUp and ModDown conversions as exact int8-split tcgen05 contractions
 // (conv_tc.cu); chunk = targets per MMA (32 or 16)
-bool conv_tc_eligible(const DevCtx& ctx);   // shapes the kernels handle
-bool conv_tc_supported(const DevCtx& ctx);  // eligible and the B tables built
+bool conv_tc_eligible(const DevCtx& ctx, uint64_t smallest);  // shapes and moduli the kernels handle
+bool conv_tc_supported(const DevCtx& ctx);                     // eligible and the B tables built
 // byte offsets of the per-(level, digit) and per-(level, fused) B matrices
 size_t conv_tc_table_layout(const DevCtx& ctx, std::vector<uint64_t>& offs);
 void conv_tc_build_tables(const DevCtx& ctx, cudaStream_t st);

@@ -55,3 +55,24 @@ def test_mixed_prime_sizes_bitexact(logN, variant, conv):
         want = oc.hmult(lv, *a, *b, kb, ka, rescale=True)
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), lv
     assert device_status(cc) == 0
+
+
+@pytest.mark.parametrize("small", ["q", "p"])
+def test_moduli_below_17_bits_leave_the_tensor_cores(small):
+    """The tensor-core reduction needs moduli above 2^17: with a smaller one among
+    the ciphertext or the special moduli its variants are refused and every other
+    one is exact."""
+    from pyfideslib_b200._capi import lib
+
+    cc, oc = _pair(9, [50, 40, 16 if small == "q" else 30, 18, 45], [60, 59, 14 if small == "p" else 58], 3)
+    for conv in (3, 4):
+        assert lib.fides_set_conv_accumulator(cc._h, conv) != 0
+    kb, ka = rand_key(oc, 7)
+    cc.upload_relin_key(kb, ka)
+    for conv in (-1, 0, 2):
+        assert lib.fides_set_conv_accumulator(cc._h, conv) == 0
+        for lv in (4, 3, 2, 1):
+            a, b = rand_ct(oc, lv, 40 + lv), rand_ct(oc, lv, 50 + lv)
+            got = cc.EvalMult(cc.upload(*a), cc.upload(*b), rescale=True).download()
+            want = oc.hmult(lv, *a, *b, kb, ka, rescale=True)
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), (conv, lv)
