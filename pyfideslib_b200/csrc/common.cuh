@@ -87,7 +87,10 @@ struct DevCtx {
 // (launch_pdl, kernels.hpp).  A kernel reads or writes nothing that an earlier
 // kernel produces or uses before pdl_wait (only context tables and switching
 // keys' addresses), and every CTA passes pdl_wait, so completion stays
-// transitive along the stream.
+// transitive along the stream.  What an earlier kernel can produce is read by
+// plain loads alone: __ldg and const __restrict__ promise data that does not
+// change while the kernel lives, which now begins before its predecessor ends, and
+// such loads may be moved above the wait.  They are for context tables.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 #endif

@@ -58,8 +58,7 @@ __device__ __forceinline__ void conv_store(uint64_t* out, const ACC& a, const AC
 // the autotuner picks per context (identical sums).
 template <int MAXIN, class ACC>
 __global__ void __launch_bounds__(kConvThreads) k_modup_conv(const __grid_constant__ DevCtx ctx, int level,
-                                                             const uint64_t* __restrict__ xt,
-                                                             uint64_t* __restrict__ dig, size_t dig_stride,
+                                                             const uint64_t* xt, uint64_t* dig, size_t dig_stride,
                                                              size_t bstride) {
     pdl_trigger();
     pdl_wait();
@@ -123,8 +122,7 @@ __global__ void __launch_bounds__(kConvThreads) k_modup_conv(const __grid_consta
 // registers of k_modup_conv (twice the resident warps), the same products.
 template <int MAXIN>
 __global__ void __launch_bounds__(kConvThreads) k_modup_conv_c1(const __grid_constant__ DevCtx ctx, int level,
-                                                                const uint64_t* __restrict__ xt,
-                                                                uint64_t* __restrict__ dig, size_t dig_stride,
+                                                                const uint64_t* xt, uint64_t* dig, size_t dig_stride,
                                                                 size_t bstride) {
     pdl_trigger();
     pdl_wait();
@@ -583,9 +581,9 @@ __global__ void __launch_bounds__(kConvThreads) k_moddown_conv(const __grid_cons
     __shared__ ulonglong2 sPinv[kConvTargets];
     const int half = blockIdx.z & 1;
     const size_t boff = (size_t)(blockIdx.z >> 1) * args.bstride;
-    const uint64_t* __restrict__ y = args.y[half] + boff;
-    uint64_t* __restrict__ w = args.w[half] + boff;
-    const uint64_t* __restrict__ ttop = args.ttop[half] ? args.ttop[half] + boff : nullptr;
+    const uint64_t* y = args.y[half] + boff;
+    uint64_t* w = args.w[half] + boff;
+    const uint64_t* ttop = args.ttop[half] ? args.ttop[half] + boff : nullptr;
     const int K = ctx.K, L = ctx.L;
     const int nout = ttop ? level : level + 1;
     const int q0 = blockIdx.y * kConvTargets;
@@ -855,7 +853,7 @@ __global__ void __launch_bounds__(128) k_dot_pt(const __grid_constant__ DevCtx c
     }
     auto term = [&](int k, ulonglong2& w, ulonglong2& x, ulonglong2& y) {
         const int b = args.baby[k];
-        w = __ldg(reinterpret_cast<const ulonglong2*>(args.p[k] + i));
+        w = *reinterpret_cast<const ulonglong2*>(args.p[k] + i);
         x = *reinterpret_cast<const ulonglong2*>(args.c0[b] + i);
         y = *reinterpret_cast<const ulonglong2*>(args.c1[b] + i);
     };
@@ -956,9 +954,8 @@ void launch_lincomb(const DevCtx& ctx, int nlimbs, const LinArgs& args, cudaStre
 // X^k in evaluation form: slot i of prime j holds psi_j^e, e = (2 brev(i) + 1) k
 // mod 2N; psi^m = fwd_tw[j][brev(m)] for m < N and psi^N = -1.
 // Role in the reference: Ciphertext::multMonomial (used by Bootstrap.cu:268).
-__global__ void k_mult_monomial(const __grid_constant__ DevCtx ctx, const uint64_t* __restrict__ in0,
-                                const uint64_t* __restrict__ in1, uint64_t* __restrict__ out0,
-                                uint64_t* __restrict__ out1, uint32_t k) {
+__global__ void k_mult_monomial(const __grid_constant__ DevCtx ctx, const uint64_t* in0, const uint64_t* in1,
+                                uint64_t* out0, uint64_t* out1, uint32_t k) {
     pdl_trigger();
     pdl_wait();
     const int limb = blockIdx.y;
@@ -984,8 +981,8 @@ void launch_mult_monomial(const DevCtx& ctx, int nlimbs, const uint64_t* in0, co
     launch_pdl(k_mult_monomial, g, 256, 0, st, ctx, in0, in1, out0, out1, k);
 }
 
-__global__ void k_automorph(const __grid_constant__ DevCtx ctx, const uint64_t* __restrict__ in,
-                            uint64_t* __restrict__ out, uint32_t galois_inv) {
+__global__ void k_automorph(const __grid_constant__ DevCtx ctx, const uint64_t* in, uint64_t* out,
+                            uint32_t galois_inv) {
     pdl_trigger();
     pdl_wait();
     const size_t base = (size_t)blockIdx.y * ctx.N;
