@@ -264,7 +264,6 @@ template <int CK, int CHUNK, bool MD>
 __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
     k_conv_tc(const __grid_constant__ DevCtx ctx, int level, const __grid_constant__ TcArgs args) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    pdl_trigger();
     const int tlog = ctx.logN - 7, ntiles = 1 << tlog;  // tiles of kTcRows = 2^7 coefficients
     // ModDown with the top limb (target 0 = prime `level`); both halves alike
     const bool fused = MD && args.md.ttop[0] != nullptr;
@@ -340,6 +339,12 @@ __global__ void __launch_bounds__(kTcThreads, CHUNK == 16 ? 3 : 2)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tslot;
+    // The next kernel of the stream may start only now.  A CTA that waits for
+    // columns then holds none, and one that holds some and waits (pdl_wait) has only
+    // kernels before it whose CTAs all hold theirs: whatever else asks for
+    // columns on this SM (a context with 32 targets per MMA beside one with 16 may
+    // want more than its 512), every holder ends and gives them back.
+    pdl_trigger();
 
     const int quarter = warp & 3, wh = warp >> 2;
     const int row = quarter * 32 + lane;

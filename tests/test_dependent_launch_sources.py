@@ -1,6 +1,8 @@
 """Source rules of the kernels that may start before their predecessor ends (those
 that call pdl_wait): their data is read by plain loads (no __restrict__, no
-__ldg but of context tables), since a read-only load may be moved above the wait."""
+__ldg but of context tables), since a read-only load may be moved above the wait,
+and the kernel that takes tensor memory lets its successor start only then: no CTA
+that a holder of columns waits for is still waiting for some itself."""
 import os
 import re
 
@@ -53,3 +55,13 @@ def test_data_is_read_by_plain_loads(name):
     for m in re.finditer(r"\b(__ldg|ldg2)\(", src):
         arg = re.sub(r"^reinterpret_cast<[^>]*>\(", "", src[m.end():m.end() + 80])
         assert arg.startswith(tables), arg
+
+
+def test_successors_start_after_tensor_memory_is_taken():
+    src = _source("conv_tc.cu")
+    assert src.count("tcgen05.alloc") == 1 and src.count("pdl_trigger();") == 1
+    (body,) = [src[a:b] for k, a, b in _kernels(src) if k == "k_conv_tc"]
+    alloc, trigger = body.index("tcgen05.alloc"), body.index("pdl_trigger();")
+    assert alloc < body.index("__syncthreads();", alloc) < trigger
+    # every CTA that allocates also frees
+    assert "return;" not in body[alloc:] and body.count("tcgen05.dealloc") == 1
