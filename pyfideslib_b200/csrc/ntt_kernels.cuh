@@ -197,7 +197,7 @@ __device__ __forceinline__ void fp_inv(uint64_t (&x)[16], Get get, double p, dou
 // ---- geometry ----
 // Every kernel has two instances: one held to 80 registers, 24 warps per SM, and
 // a wide one of up to 128 registers for launches that do not fill the SMs anyway
-// (kWideThreads): with all the loads of a thread in flight and no spills its
+// (wide_threads): with all the loads of a thread in flight and no spills its
 // warps are shorter, which is all that counts there.
 constexpr int min_ctas(int nt, bool wide) {
     const int c = (wide ? 512 : 768) / nt;
@@ -936,11 +936,17 @@ __global__ void __launch_bounds__(ColGeo<LR, LC>::NT, WIDE ? ColGeo<LR, LC>::MIN
 // grid (tiles, batch element, limb): CTAs run x fastest, then y, so the
 // elements of a batch that share a prime run together and its twiddle table is
 // fetched from HBM once per launch rather than once per element
-// Threads up to which a launch takes the wide instances: what the narrow ones
-// hold in one wave.  N = 2^16, 50-bit limbs, narrow / wide: 18 limbs 15.0 / 11.2 us
-// forward, 24 limbs 14.8 / 15.3, 29 limbs 17.0 / 18.2; N = 2^15, 59-bit limbs, 2 x 20
-// limbs 25.1 / 22.2, 2 x 29 limbs 28.7 / 29.1.
-constexpr size_t kWideThreads = (size_t)768 * 148;
+// Threads up to which a launch takes the wide instances, where the two curves
+// cross (back to back, medians of five; 65536 words are 4096 threads).  Forward
+// and the short columns' inverse: 640 threads per SM, 23.1 x 65536 words.  us
+// narrow / wide: N = 2^16, 50 bits, forward 18 limbs 14.9 / 11.3, 23 limbs 15.0 / 14.4,
+// 24 limbs 15.0 / 15.4, 27 limbs 14.8 / 15.6; 59 bits 23 limbs 27.4 / 26.0, 24 limbs
+// 27.8 / 27.7, 27 limbs 27.5 / 28.1; N = 2^13 23 x 65536 words forward 13.3 / 12.0 and
+// inverse 14.2 / 12.6, 25 x forward 13.2 / 13.4 and inverse 14.2 / 14.4.  The inverse
+// with columns of 128 words and more stays ahead up to one narrow wave, 768 threads
+// per SM: 2^16 50 bits 24 limbs 16.4 / 16.0, 27 limbs 16.3 / 16.3; 2^15 59 bits 2 x 24
+// limbs 28.4 / 26.4, 2 x 27 limbs 28.8 / 26.5.
+constexpr size_t wide_threads(bool inverse, int lr) { return (size_t)(inverse && lr >= 7 ? 768 : 640) * 148; }
 
 template <int LR, int LC>
 struct NttN {
@@ -949,30 +955,30 @@ struct NttN {
     static dim3 gcols(const LimbMap& m) { return dim3(CG::C / CG::TC, m.nb > 0 ? m.nb : 1, m.total); }
     static dim3 grows(const LimbMap& m) { return dim3(RG::GROUPS / RG::W, m.nb > 0 ? m.nb : 1, m.total); }
 
-    template <class K>
+    template <bool INV, class K>
     static void launch(K narrow, K wide, dim3 g, int nt, const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
-        launch_pdl((size_t)g.x * g.y * g.z * nt <= kWideThreads ? wide : narrow, g, nt, 0, st, ctx, map);
+        launch_pdl((size_t)g.x * g.y * g.z * nt <= wide_threads(INV, LR) ? wide : narrow, g, nt, 0, st, ctx, map);
     }
     static void fwd_cols(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
         if (ntt_fwd_is_fp(ctx.ntt_variant))
-            launch(k_ntt_fwd_cols<LR, LC, true, false>, k_ntt_fwd_cols<LR, LC, true, true>, gcols(map), CG::NT, ctx, map, st);
+            launch<false>(k_ntt_fwd_cols<LR, LC, true, false>, k_ntt_fwd_cols<LR, LC, true, true>, gcols(map), CG::NT, ctx, map, st);
         else
-            launch(k_ntt_fwd_cols<LR, LC, false, false>, k_ntt_fwd_cols<LR, LC, false, true>, gcols(map), CG::NT, ctx, map, st);
+            launch<false>(k_ntt_fwd_cols<LR, LC, false, false>, k_ntt_fwd_cols<LR, LC, false, true>, gcols(map), CG::NT, ctx, map, st);
     }
     static void fwd(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
         fwd_cols(ctx, map, st);
         if (ntt_fwd_is_fp(ctx.ntt_variant))
-            launch(k_ntt_fwd_rows<LR, LC, true, false>, k_ntt_fwd_rows<LR, LC, true, true>, grows(map), RG::NT, ctx, map, st);
+            launch<false>(k_ntt_fwd_rows<LR, LC, true, false>, k_ntt_fwd_rows<LR, LC, true, true>, grows(map), RG::NT, ctx, map, st);
         else
-            launch(k_ntt_fwd_rows<LR, LC, false, false>, k_ntt_fwd_rows<LR, LC, false, true>, grows(map), RG::NT, ctx, map, st);
+            launch<false>(k_ntt_fwd_rows<LR, LC, false, false>, k_ntt_fwd_rows<LR, LC, false, true>, grows(map), RG::NT, ctx, map, st);
     }
     static void inv(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
         if (ntt_inv_is_fp(ctx.intt_variant)) {
-            launch(k_ntt_inv_rows<LR, LC, true, false>, k_ntt_inv_rows<LR, LC, true, true>, grows(map), RG::NT, ctx, map, st);
-            launch(k_ntt_inv_cols<LR, LC, true, false>, k_ntt_inv_cols<LR, LC, true, true>, gcols(map), CG::NT, ctx, map, st);
+            launch<true>(k_ntt_inv_rows<LR, LC, true, false>, k_ntt_inv_rows<LR, LC, true, true>, grows(map), RG::NT, ctx, map, st);
+            launch<true>(k_ntt_inv_cols<LR, LC, true, false>, k_ntt_inv_cols<LR, LC, true, true>, gcols(map), CG::NT, ctx, map, st);
         } else {
-            launch(k_ntt_inv_rows<LR, LC, false, false>, k_ntt_inv_rows<LR, LC, false, true>, grows(map), RG::NT, ctx, map, st);
-            launch(k_ntt_inv_cols<LR, LC, false, false>, k_ntt_inv_cols<LR, LC, false, true>, gcols(map), CG::NT, ctx, map, st);
+            launch<true>(k_ntt_inv_rows<LR, LC, false, false>, k_ntt_inv_rows<LR, LC, false, true>, grows(map), RG::NT, ctx, map, st);
+            launch<true>(k_ntt_inv_cols<LR, LC, false, false>, k_ntt_inv_cols<LR, LC, false, true>, gcols(map), CG::NT, ctx, map, st);
         }
     }
 

@@ -30,7 +30,7 @@ def _kernels(src):
 @pytest.mark.parametrize("name", FILES)
 def test_early_kernels_wait(name):
     src = _source(name)
-    launched = set(re.findall(r"launch(?:_pdl)?\(\s*(k_\w+)", src))
+    launched = set(re.findall(r"launch(?:_pdl)?(?:<\w+>)?\(\s*(k_\w+)", src))
     waiting = {k for k, a, b in _kernels(src) if src[a:b].count("pdl_wait();") == 1}
     assert launched and launched <= waiting, launched - waiting
 

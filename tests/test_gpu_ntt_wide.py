@@ -1,6 +1,6 @@
-"""The transforms' wide instances (launches of at most 768 threads per SM, one thread
-per 16 coefficients) and narrow ones: bit-exact against the oracle on each side of
-the line, with the prologues and epilogues the library uses (products, rescale,
+"""The transforms' wide instances (launches of at most 640 or 768 threads per SM, one
+thread per 16 coefficients) and narrow ones: bit-exact against the oracle on each side
+of both lines, with the prologues and epilogues the library uses (products, rescale,
 ModUp / ModDown scales through a rotation)."""
 import numpy as np
 import pytest
@@ -16,8 +16,8 @@ def test_wide_and_narrow_bitexact(logN, variant):
     cc, oc = make_pair(logN, 3, 1, 2)
     cc.set_ntt_variant(variant)
     pid = list(range(4))
-    edge = 768 * 148 * 16 // (4 * cc.N)  # polynomials of 4 limbs up to the line
-    for npoly in (1, edge, edge + 1):
+    lines = [t * 148 * 16 // (4 * cc.N) for t in (640, 768)]  # polynomials of 4 limbs up to each line
+    for npoly in (1, lines[0], lines[0] + 1, lines[1], lines[1] + 1):
         x = np.stack([oc.random(pid, 10 * logN + k) for k in range(npoly)])
         for i in pid:
             x[-1, i] = oc.primes[i] - 1
