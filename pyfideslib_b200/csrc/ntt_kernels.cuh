@@ -737,7 +737,10 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, MB)
 // ---------------------------------------------------------------------------
 // Prologue modes of the inverse row pass (per segment): IL_PLAIN reads `in`,
 // IL_MUL the product in*in2.
-template <int LR, int LC, bool FP, bool WIDE>
+// ODD: the limbs may start at an odd word, as a caller's of fides_ntt and
+// fides_ntt_batch (an odd stride) may; IL_PLAIN, 8-byte loads.  An instance of its own:
+// the choice made in the kernel cost an affine step at N = 2^14 0.25 of 68.4 us.
+template <int LR, int LC, bool FP, bool WIDE, bool ODD = false>
 __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, WIDE ? RowGeo<LR, LC>::MINB_WIDE : RowGeo<LR, LC>::MINB)
     k_ntt_inv_rows(const __grid_constant__ DevCtx ctx, const __grid_constant__ LimbMap map) {
     using G = RowGeo<LR, LC>;
@@ -769,9 +772,7 @@ __global__ void __launch_bounds__(RowGeo<LR, LC>::NT, WIDE ? RowGeo<LR, LC>::MIN
     const double p = __ull2double_rn(pc.p), pinv = as_f64(pc.pinv_f64);
     pdl_wait();
     uint64_t x[16];
-    if (reinterpret_cast<uintptr_t>(lr.in) & 15) {
-        // a caller's limbs may start at an odd word (fides_ntt, fides_ntt_batch
-        // with an odd stride; always IL_PLAIN): 8-byte loads, one by one
+    if constexpr (ODD) {
 #pragma unroll 1
         for (int i = lane; i < G::GW; i += G::WL) {
             const uint64_t u = lr.in[base + i];
@@ -972,12 +973,25 @@ struct NttN {
         else
             launch<false>(k_ntt_fwd_rows<LR, LC, false, false>, k_ntt_fwd_rows<LR, LC, false, true>, grows(map), RG::NT, ctx, map, st);
     }
+    static bool odd_words(const LimbMap& m) {
+        bool odd = false;
+        for (int s = 0; s < m.nseg; ++s)
+            odd = odd || (reinterpret_cast<uintptr_t>(m.seg[s].in) & 15) || (m.nb > 1 && (m.seg[s].bstride & 1));
+        return odd;
+    }
     static void inv(const DevCtx& ctx, const LimbMap& map, cudaStream_t st) {
+        const bool odd = odd_words(map);
         if (ntt_inv_is_fp(ctx.intt_variant)) {
-            launch<true>(k_ntt_inv_rows<LR, LC, true, false>, k_ntt_inv_rows<LR, LC, true, true>, grows(map), RG::NT, ctx, map, st);
+            if (odd)
+                launch_pdl(k_ntt_inv_rows<LR, LC, true, false, true>, grows(map), RG::NT, 0, st, ctx, map);
+            else
+                launch<true>(k_ntt_inv_rows<LR, LC, true, false>, k_ntt_inv_rows<LR, LC, true, true>, grows(map), RG::NT, ctx, map, st);
             launch<true>(k_ntt_inv_cols<LR, LC, true, false>, k_ntt_inv_cols<LR, LC, true, true>, gcols(map), CG::NT, ctx, map, st);
         } else {
-            launch<true>(k_ntt_inv_rows<LR, LC, false, false>, k_ntt_inv_rows<LR, LC, false, true>, grows(map), RG::NT, ctx, map, st);
+            if (odd)
+                launch_pdl(k_ntt_inv_rows<LR, LC, false, false, true>, grows(map), RG::NT, 0, st, ctx, map);
+            else
+                launch<true>(k_ntt_inv_rows<LR, LC, false, false>, k_ntt_inv_rows<LR, LC, false, true>, grows(map), RG::NT, ctx, map, st);
             launch<true>(k_ntt_inv_cols<LR, LC, false, false>, k_ntt_inv_cols<LR, LC, false, true>, gcols(map), CG::NT, ctx, map, st);
         }
     }
