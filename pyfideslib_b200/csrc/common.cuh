@@ -10,7 +10,7 @@ namespace fides {
 
 constexpr int kMaxPrimes = 128;
 constexpr int kMaxSeg = 8;
-constexpr int kMaxBatch = 32;  // ciphertexts per batched launch (blockIdx.z)
+constexpr int kMaxBatch = 32;  // ciphertexts per batched launch
 
 // Bits of a context's device error word (DevCtx::err).  A kernel whose
 // bounded wait gives up sets its bit and leaves invalid outputs; the next
@@ -119,7 +119,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 struct LimbMap {
     int nseg;
     int total;
-    int nb;  // batch elements (gridDim.z); 0 means 1
+    int nb;  // batch elements (gridDim.y); 0 means 1
     LimbSeg seg[kMaxSeg];
     uint64_t* bout[2][kMaxBatch];
     const uint64_t* bin[2][kMaxBatch];

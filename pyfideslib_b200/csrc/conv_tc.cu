@@ -116,9 +116,9 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 // floor(V'/2^16) = floor(e/2^16) + o  and  V' mod 2^64 = e + (o << 16).
 // V' < 8 cnt 255 p (cnt input limbs): the quotient has at most 15 bits, so 32
 // bits T = floor(V' / 2^s) of V' and one 32-bit high product give it,
-//   q = floor(T M / 2^(32+k)),  M = floor(2^(32+k+s) / p) or one less,
+//   q = floor(T M / 2^(32+k)),  M = floor(2^(32+k+s) / p) or up to two less,
 // with s = max(16, bits(p) + bits(2040 cnt) - 32), k = bits(p) - 1 - s: short of
-// V'/p by less than 1 + 2^s / p + 2 T / 2^(32+k) < 2, so V' - q p (formed modulo
+// V'/p by less than 1 + 2^s / p + 3 T / 2^(32+k) < 2, so V' - q p (formed modulo
 // 2^64) lies in [0, 2p).  (A 64-bit Barrett quotient, floor(2^80 / p), took
 // eight half-rate multiplies per output against three, and that pipe was 65%
 // busy: ModUp of 32 elements 608 us, ModDown 598 us at the HMult shape.)

@@ -4,7 +4,7 @@
 // magnitude are exact).  A product y w = h + l is split exactly by an FMA
 // (h = fl(y w), l = fma(y, w, -h)); a quotient estimate q, rounded to an
 // integer through the 1.5 * 2^52 shift (valid while |q| < 2^51), gives the
-// remainder fma(-q, p, h) + l exactly.  Used by the NTT butterflies (ntt.cu)
+// remainder fma(-q, p, h) + l exactly.  Used by the NTT butterflies (ntt_kernels.cuh)
 // and the key-switch inner product (ks.cu); the integer pipes that the 64-bit
 // Shoup/Barrett forms keep busy are left free.
 #pragma once
@@ -40,7 +40,7 @@ __device__ __forceinline__ double fp_mulw_sh(double y, double w, double wq, doub
     return __dadd_rn(__fma_rn(-q, p, h), l);
 }
 
-// x - rint(x / p) p, magnitude <= p/2 + |x| 2^-52 (|x| < 2^51)
+// x - rint(x / p) p, magnitude <= p/2 + |x| 2^-52 (|x| < 2^53)
 __device__ __forceinline__ double fp_center(double x, double p, double pinv) {
     const double q = __dsub_rn(__fma_rn(x, pinv, kRint), kRint);
     return __fma_rn(-q, p, x);

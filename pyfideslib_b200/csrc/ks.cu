@@ -224,9 +224,10 @@ void launch_modup_conv(const DevCtx& ctx, int level, int nb, const uint64_t* xt,
 // from L2 to the rest of the batch.  (Folding the element into blockIdx.x and
 // dividing by the batch size per thread cost 32 hoisted rotations 1.1%.)
 // FPK: limbs of primes below 2^50 accumulate on the FP64 pipes (fp64.cuh):
-// each product x k is reduced to |r| <= 0.875p, the sum of up to 8 digits
-// stays below 7p < 2^53, and one centring plus a floor reduction give the
-// canonical residue -- the same values as the 128-bit integer sums.
+// each product x k is reduced to |r| <= 0.875p, the sum of up to 6 digits (more
+// take the integer sums) and of the P c0 term stays below 5.8p < 2^53, and one
+// centring plus a floor reduction give the canonical residue -- the same values
+// as the 128-bit integer sums.
 // SEED: some element's key is seeded (ka null), its a half regenerated per
 // coefficient; the instantiation without it carries no generator code (52
 // registers; 48 measured the same).  Left free, the unrolled digit loop with
@@ -405,7 +406,11 @@ void launch_ks_inner(const DevCtx& ctx, int level, int nb, const KsArgs& args, c
 // and the ciphertext limbs leave as e + P^-1 x,
 //   XB[m] = a0 b0 + P^-1 sum_d D_d[t] kb[d][t]
 //   XA[m] = a0 b1 + a1 b0 + P^-1 sum_d D_d[t] ka[d][t]      (m < n),
-// the special limbs as the sums.  Bounds and sums as in k_ks_inner.
+// the special limbs as the sums.  FP64 limbs, up to 8 digits: the own digit's
+// product is signed, |a1 b1 mod| <= 0.875p, so each digit's product with the key is
+// too, the sum is at most 7p < 2^53, and centred, times P^-1 (0.54p) and with the
+// one or two products added it stays below 2.3p.  (tests/test_exact_arith.py runs
+// these sums on the host.)  Integer sums as in k_ks_inner.
 // ---------------------------------------------------------------------------
 // Its loads' latency bounds this kernel (8 pairs: 8 of 16 stall cycles per
 // instruction, DRAM 53%).

@@ -63,8 +63,9 @@ struct Tab {
     std::vector<double> c, q;
 };
 
-/* pattern 0 random, 1 all p - 1, 2 alternating 0 / p - 1, 3 all 0; returns
- * the number of wrong residues, -1 when a bound is broken */
+/* pattern 0 random, 1 all p - 1, 2 alternating 0 / p - 1, 3 all 0; the inverse runs
+ * from canonical residues and from centred ones (what a product in its load
+ * leaves).  Returns the number of wrong residues, -1 when a bound is broken */
 extern "C" int emu_sched_check(int logn, uint64_t p, uint64_t psi, uint64_t seed, int pattern) {
     using namespace fides;
     const int lr = logn / 2, lc = logn - lr, N = 1 << logn;
@@ -130,8 +131,6 @@ extern "C" int emu_sched_check(int logn, uint64_t p, uint64_t psi, uint64_t seed
     int bad = 0;
     for (int j = 0; j < N; ++j) bad += pos_to_u(d[j], pd, pinv) != e[j];
     if (g_bad) return -1;
-    /* inverse */
-    for (int j = 0; j < N; ++j) d[j] = (double)e[j];
     const InvSched iv = inv_sched(lr, lc);
     const uint64_t ninv = powmod(N, p - 2, p), s1 = mulmod(ninv, v.w[1], p);
     auto group = [&](const InvGroup& G, int bit0, int nst, bool formed) {
@@ -152,16 +151,19 @@ extern "C" int emu_sched_check(int logn, uint64_t p, uint64_t psi, uint64_t seed
             }
         }
     };
-    if (lc > 4) group(iv.ra, 0, lc - 4, true);
-    group(iv.rb, lc - 4, 4, false);
-    if (lr > 4) group(iv.ca, lc, lr - 4, false);
-    group(iv.cb, lc + lr - 4, 3, false);
     auto cst = [&](uint64_t c) { return c > p / 2 ? -(double)(p - c) : (double)c; };
     const double a0 = cst(ninv), a1 = cst(s1), a0q = a0 * pinv, a1q = a1 * pinv;
-    for (int j = 0; j < N / 2; ++j) {
-        const double x = d[j], y = d[j + N / 2];
-        bad += pos_to_u(mulw(x + y, a0, a0q, pd, kRint + 2.0), pd, pinv) != a[j];
-        bad += pos_to_u(mulw(x - y, a1, a1q, pd, kRint + 2.0), pd, pinv) != a[j + N / 2];
+    for (int centred = 0; centred < 2; ++centred) {
+        for (int j = 0; j < N; ++j) d[j] = centred && e[j] > p / 2 ? -(double)(p - e[j]) : (double)e[j];
+        if (lc > 4) group(iv.ra, 0, lc - 4, true);
+        group(iv.rb, lc - 4, 4, false);
+        if (lr > 4) group(iv.ca, lc, lr - 4, false);
+        group(iv.cb, lc + lr - 4, 3, false);
+        for (int j = 0; j < N / 2; ++j) {
+            const double x = d[j], y = d[j + N / 2];
+            bad += pos_to_u(mulw(x + y, a0, a0q, pd, kRint + 2.0), pd, pinv) != a[j];
+            bad += pos_to_u(mulw(x - y, a1, a1q, pd, kRint + 2.0), pd, pinv) != a[j + N / 2];
+        }
     }
     return g_bad ? -1 : bad;
 }

@@ -1,27 +1,27 @@
 """CPU checks of the exactness arguments behind the FP64 and tensor-core paths.
 
 The CUDA kernels compute the same residues as the integer arithmetic only
-because of value bounds (fp64.cuh, ntt.cu, conv_tc.cu).  These tests restate
-the device arithmetic on the host and run it against exact integer
-arithmetic on the cases the bounds are tight for:
+because of value bounds (fp64.cuh, ks.cu, conv_tc.cu; the transforms' in
+test_ntt_sched.py).  These tests restate the device arithmetic on the host and
+run it against exact integer arithmetic on the cases the bounds are tight for
+(tests/exact_arith_emu.c, C99 fma):
 
-* the double-precision NTT with the kernels' stage schedule (column pass
-  centring on odd stages, row pass on even ones, doubles passed between the
-  passes, one floor reduction at the end; inverse with centred sums) on primes
-  just below 2^50, random residues, p-1 everywhere and alternating 0/p-1
-  (tests/exact_arith_emu.c, C99 fma);
-* the FP64 key-switch sums of up to 8 digit products, including maximal
-  operands, and the tensor product's single products and sums of two
-  (floor-reduced without centring);
+* the FP64 key-switch sums of rotations, and of products with their tensor
+  product: up to 8 digits, the signed own-digit product, digit values as the
+  row pass leaves them, maximal operands;
+* the FP64 plaintext dot products in runs of seven, and element-wise products;
 * the int8-split conversion: byte layout of A and B in the canonical K-major
   shared-memory form, the matrix product of the tensor-core MMAs, the
-  reassembly of V' and its one-correction Barrett step (numpy / Python ints).
+  reassembly of V' and its reduction by a 32-bit quotient for every prime size
+  and digit size, the lift of a dropped top limb (numpy / Python ints).
 The GPU parity tests then check the kernels themselves against the oracle.
 """
 import ctypes
+import math
 import os
 import random
 import subprocess
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -75,59 +75,74 @@ def emu(tmp_path_factory):
     subprocess.run(["gcc", "-O2", "-ffp-contract=off", "-frounding-math", "-shared", "-fPIC",
                     os.path.join(HERE, "exact_arith_emu.c"), "-o", out, "-lm"], check=True)
     lib = ctypes.CDLL(out)
-    lib.emu_ntt_check.argtypes = [ctypes.c_uint64, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
-    lib.emu_ntt_gen_check.argtypes = [ctypes.c_uint64, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
-    lib.emu_ntt_sg_check.argtypes = [ctypes.c_uint64, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int]
-    lib.emu_ks_check.argtypes = [ctypes.c_uint64, ctypes.c_int, ctypes.c_uint64, ctypes.c_int, ctypes.c_int]
-    lib.emu_tensor_check.argtypes = [ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int, ctypes.c_int]
+    u64, i32 = ctypes.c_uint64, ctypes.c_int
+    lib.emu_ks_check.argtypes = [u64, i32, i32, u64, i32, i32]
+    lib.emu_hmult_check.argtypes = [u64, i32, i32, i32, u64, i32, i32]
+    lib.emu_dot_check.argtypes = [u64, i32, i32, u64, i32, i32]
     return lib
 
 
 PRIMES_50 = _ntt_primes(1 << 50, 3) + _ntt_primes((1 << 49) + (1 << 47), 1)
 
 
-@pytest.mark.parametrize("p", PRIMES_50)
-def test_fp64_ntt_schedule_exact(emu, p):
-    psi = _psi(p)
-    for pattern in (0, 1, 2):
-        assert emu.emu_ntt_check(p, psi, 1000 + pattern, pattern) == 0, pattern
-
-
-@pytest.mark.parametrize("p", PRIMES_50)
-def test_fp64_ntt_generated_row_twiddles_exact(emu, p):
-    """Forward variant 9: the row pass forms its twiddles on the fly and
-    takes their quotient companions as fl(w * pinv) (not correctly rounded),
-    centring X at every row stage."""
-    psi = _psi(p)
-    for pattern in (0, 1, 2):
-        assert emu.emu_ntt_gen_check(p, psi, 2000 + pattern, pattern) == 0, pattern
-
-
-@pytest.mark.parametrize("p", PRIMES_50)
-def test_fp64_ntt_staged_generated_row_twiddles_exact(emu, p):
-    """Forward variant 9 and its inverse configuration: exact staged twiddles
-    for the forward row pass's first four stages, products of a table entry
-    and psi_br[g] (unreduced, sloppy quotient companion) for the last four,
-    which centre X at every stage; the inverse row pass forms its per-thread
-    twiddles the same way."""
-    psi = _psi(p)
-    for pattern in (0, 1, 2):
-        assert emu.emu_ntt_sg_check(p, psi, 3000 + pattern, pattern) == 0, pattern
-
-
 @pytest.mark.parametrize("p", PRIMES_50[:2])
 def test_fp64_keyswitch_sums_exact(emu, p):
-    for nd in range(1, 9):
-        assert emu.emu_ks_check(p, nd, nd, 20000, 0) == 0, nd
-        assert emu.emu_ks_check(p, nd, nd, 4, 1) == 0, nd
+    for nd in range(1, 7):
+        for c0 in (0, 1):
+            assert emu.emu_ks_check(p, nd, c0, nd, 20000, 0) == 0, nd
+            assert emu.emu_ks_check(p, nd, c0, nd, 4, 1) == 0, nd
 
 
 @pytest.mark.parametrize("p", PRIMES_50)
-def test_fp64_tensor_products_exact(emu, p):
-    """e0 = a0 b0 and e1 = a0 b1 + a1 b0 as k_tensor forms them on the FP64
-    pipes: products reduced to |r| <= 0.875p, floor-reduced without centring."""
-    assert emu.emu_tensor_check(p, 7, 100000, 0) == 0
-    assert emu.emu_tensor_check(p, 7, 4, 1) == 0
+def test_fp64_product_sums_exact(emu, p):
+    """Up to 8 digits in the kernel of its own, up to 6 fused into the row pass
+    (lazy digit values); own: the digit of the limb, -1 for a special limb."""
+    for lazy in (0, 1):
+        for nd in range(1, 7 if lazy else 9):
+            for own in range(-1, nd):
+                assert emu.emu_hmult_check(p, nd, own, lazy, 10 * nd + own, 2000, 0) == 0, (lazy, nd, own)
+                assert emu.emu_hmult_check(p, nd, own, lazy, 1, 16, 1) == 0, (lazy, nd, own)
+
+
+@pytest.mark.parametrize("p", PRIMES_50)
+def test_fp64_dot_products_exact(emu, p):
+    for n in (1, 6, 7, 8, 15, 64):
+        for accumulate in (0, 1):
+            assert emu.emu_dot_check(p, n, accumulate, n, 2000, 0) == 0, n
+            assert emu.emu_dot_check(p, n, accumulate, n, 2, 1) == 0, n
+
+
+M32, M64 = (1 << 32) - 1, (1 << 64) - 1
+
+
+def _tc_mod(p, cnt):
+    """conv_tc.cu tc_mod: (s, k, M), from the context's double 1/p (rounded up below 2^50)."""
+    inv = 1.0 / float(p)
+    if p < 1 << 50 and Fraction(inv) * p < 1:
+        inv = math.nextafter(inv, 1.0)
+    bits = p.bit_length()
+    s = max(16, bits + (2040 * cnt).bit_length() - 32)
+    k = max(0, bits - 1 - s)
+    m = int(math.ldexp(inv, 32 + k + s))
+    assert 0 < m - 1 <= M32  # the device's 32 bits hold it
+    return s, k, m - 1
+
+
+def _reduce_cols(c, p, mod):
+    """conv_tc.cu reduce_cols in 32- and 64-bit words."""
+    s, k, M = mod
+    w = [c[2 * i] + (c[2 * i + 1] << 8) for i in range(4)]
+    assert max(w) <= M32
+    e, o = (w[2] << 32) | w[0], (w[3] << 32) | w[1]
+    h = (e >> 16) + o
+    T = h >> (s - 16)
+    assert h <= M64 and s - 16 < 32 and T <= M32
+    q = (T * M >> 32) >> k
+    np_ = -p & M64
+    a = (q * (np_ & M32) + e) & M64
+    r = (a + (((q * (np_ >> 32)) & M32) << 32) + (o << 16)) & M64
+    assert r < 2 * p, (p, q)
+    return r if r < p else r - p
 
 
 def _conv_tc_emulate(ck, cnt, ntar, bits, seed):
@@ -167,7 +182,7 @@ def _conv_tc_emulate(ck, cnt, ntar, bits, seed):
                         for r in range(nrows)])
         return buf[idx].astype(np.int64)
 
-    bad, m64 = 0, (1 << 64) - 1
+    bad = 0
     for m0 in range(0, ntar2, 32):
         nt = min(32, ntar2 - m0)
         D = np.zeros((rows, nt * 8), np.int64)
@@ -179,15 +194,9 @@ def _conv_tc_emulate(ck, cnt, ntar, bits, seed):
             if m >= ntar:
                 continue
             p = ps[m]
-            mu = (1 << 80) // p
+            mod = _tc_mod(p, cnt)
             for r in range(0, rows, 3):
-                c = [int(v) for v in D[r, mm * 8:mm * 8 + 8]]
-                w = [c[2 * k] + (c[2 * k + 1] << 8) for k in range(4)]
-                e, o = (w[2] << 32) | w[0], (w[3] << 32) | w[1]
-                q = (((e >> 16) + o) * mu) >> 64
-                res = (e + ((o << 16) & m64) - q * p) & m64
-                assert res < 2 * p
-                res = res - p if res >= p else res
+                res = _reduce_cols([int(v) for v in D[r, mm * 8:mm * 8 + 8]], p, mod)
                 bad += res != sum(x[i][r] * M[i][m] for i in range(cnt)) % p
     return bad
 
@@ -197,22 +206,53 @@ def test_tensor_conversion_layout_exact(ck, cnt, ntar, bits):
     assert _conv_tc_emulate(ck, cnt, ntar, bits, ck * 100 + ntar) == 0
 
 
-def test_tensor_conversion_barrett_bound():
-    """The reassembly and one-correction Barrett step on random and maximal
-    column sums (16 limbs x 8 bytes of 255 x 255) for 18- to 62-bit primes."""
+def _reduction_moduli():
+    """18- to 62-bit odd numbers: the least and the greatest of each width, and others."""
+    rnd = random.Random(11)
+    for bits in range(18, 63):
+        yield (1 << (bits - 1)) + 1
+        yield (1 << bits) - 1
+        yield rnd.randrange(1 << (bits - 1), 1 << bits) | 1
+
+
+def test_tensor_conversion_reduction_bound():
+    """The reassembly, the 32-bit quotient and its one correction for 18- to 62-bit
+    moduli and digits of 1 to 16 limbs: V' at its greatest (bytes of 255 against
+    constants p - 1), at multiples of p and beside them, and random."""
     rnd = random.Random(7)
-    m64 = (1 << 64) - 1
-    cmax = 16 * 8 * 255 * 255
-    for trial in range(20000):
-        c = [cmax if trial % 4 == 0 else rnd.randrange(cmax + 1) for _ in range(8)]
-        p = rnd.randrange(2 ** (rnd.choice([18, 40, 50, 60, 62]) - 1), 2 ** 62) | 1
-        p = min(p, 2 ** 62 - 1)
-        v = sum(c[s] << (8 * s) for s in range(8))
-        w = [c[2 * k] + (c[2 * k + 1] << 8) for k in range(4)]
-        e, o = (w[2] << 32) | w[0], (w[3] << 32) | w[1]
-        t = (e >> 16) + o
-        assert t == v >> 16 and t < 2 ** 64
-        q = (t * ((1 << 80) // p)) >> 64
-        r = (e + ((o << 16) & m64) - q * p) & m64
-        assert r < 2 * p
-        assert (r - p if r >= p else r) == v % p
+    for p in _reduction_moduli():
+        for cnt in (1, 2, 3, 4, 7, 10, 15, 16):
+            mod = _tc_mod(p, cnt)
+            cases = [([255] * 8 * cnt, [p - 1] * 8 * cnt), ([0] * 8 * cnt, [p - 1] * 8 * cnt),
+                     ([1] + [0] * (8 * cnt - 1), [p - 1] * 8 * cnt), ([255, 1] + [255] * (8 * cnt - 2), [p - 1, 255] * 4 * cnt),
+                     ([rnd.randrange(256) for _ in range(8 * cnt)], [rnd.randrange(p) for _ in range(8 * cnt)])]
+            for xs, ms in cases:
+                c = [sum(x * (m >> (8 * s) & 255) for x, m in zip(xs, ms)) for s in range(8)]
+                v = sum(x * m for x, m in zip(xs, ms))
+                assert v == sum(c[s] << (8 * s) for s in range(8)) and max(c) < 2 ** 23
+                assert _reduce_cols(c, p, mod) == v % p, (p, cnt)
+
+
+def test_tensor_conversion_top_limb_lift():
+    """The fused ModDown adds the centred top limb: one conditional addition where
+    the top modulus is below twice the target, else a reduction; v and tl at their
+    ends and at the centring's edge."""
+    rnd = random.Random(13)
+
+    def signed(x):
+        return x - (1 << 64) if x >> 63 else x
+
+    for p in _reduction_moduli():
+        for ql in {p + 2, 2 * p - 1, p - 2, p // 2 | 1, p // 5 | 1, 2 * p + 1, min(9 * p + 2, 2 ** 62 - 1), 2 ** 61 + 1} - {p}:
+            for tl in (0, 1, ql // 2 - 1, ql // 2, ql // 2 + 1, ql - 1, rnd.randrange(ql)):
+                for v in (0, 1, p // 2, p - 1, rnd.randrange(p)):
+                    up = tl > ql >> 1
+                    want = (v + tl - (ql if up else 0)) % p
+                    if ql < 2 * p:  # kTcNear
+                        x = (v + ((tl - ql) & M64 if up else tl) + (0 if up else -p & M64)) & M64
+                        assert ((x + p) & M64 if signed(x) < 0 else x) == want, (p, ql, tl, v)
+                    # also such a target's form beside one that is not near
+                    sw = tl + (p - ql % p if up else 0)
+                    assert sw <= M64
+                    sw = sw % p if p < ql else sw
+                    assert v + sw - (p if v + sw >= p else 0) == want, (p, ql, tl, v)

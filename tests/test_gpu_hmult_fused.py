@@ -1,6 +1,6 @@
 """HMult with the tensor product inside the key switch (no tensor kernel): against
 the oracle at every level, with and without rescale, for the integer and FP64
-arithmetics and sums, the inner product on its own or fused into the digits' row
+arithmetics and sums, one to eight digits, the inner product on its own or fused into the digits' row
 pass (in one launch or two), squares, extreme residues, and inputs at mixed levels
 in one batch."""
 import numpy as np
@@ -11,7 +11,8 @@ from gpu_helpers import device_status, make_pair, rand_ct, rand_key
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("logN,L,K,dnum", [(9, 5, 2, 3), (12, 7, 3, 3), (13, 6, 1, 6), (11, 3, 3, 1)])
+@pytest.mark.parametrize("logN,L,K,dnum", [(9, 5, 2, 3), (12, 7, 3, 3), (13, 6, 1, 6), (11, 3, 3, 1),
+                                           (10, 7, 1, 7), (12, 8, 1, 8), (9, 15, 2, 8)])
 @pytest.mark.parametrize("variant,ks", [(9, 1), (9, 0), (9, 11), (9, 3), (9, 10), (3, 1), (3, 0), (3, 11), (3, 2)])
 def test_tensor_in_key_switch_bitexact(logN, L, K, dnum, variant, ks):
     from pyfideslib_b200._capi import lib

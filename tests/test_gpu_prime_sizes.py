@@ -1,6 +1,6 @@
 """Every arithmetic a limb can take, by the size of its prime, in one context:
-61-bit and below 40-bit primes (Harvey butterflies), 40- to 60-bit ones (split
-butterflies, or the FP64 pipes below 50 bits), and the tensor-core conversions'
+primes of 56 bits and more (Harvey butterflies), smaller ones (three-product
+quotients, or the FP64 pipes below 50 bits), and the tensor-core conversions'
 reduction from 18- to 61-bit targets.  NTT and HMult + rescale bit-exact against
 the oracle, random and extreme residues, integer and FP64 variants."""
 import numpy as np
