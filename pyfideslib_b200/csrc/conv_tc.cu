@@ -33,7 +33,6 @@
 // CTA.  Every wait on the MMA completion barrier is bounded; a timeout sets an
 // error flag and the CTA releases its tensor memory and returns.
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "kernels.hpp"
@@ -503,31 +502,19 @@ size_t tc_smem_bytes(int ck, int ntar, bool md) {
 constexpr int kTcMaxTargets = 48;
 constexpr size_t kTcSmemCap = 160 * 1024;
 
-template <int CK, int CHUNK, bool MD>
-void set_smem_attr() {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        cudaFuncSetAttribute(k_conv_tc<CK, CHUNK, MD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemCap);
-    });
-}
-
 template <int CHUNK, bool MD>
 void launch_ck(int ck, dim3 g, size_t smem, const DevCtx& ctx, int level, const TcArgs& a, cudaStream_t st) {
     switch (ck) {
         case 1:
-            set_smem_attr<1, CHUNK, MD>();
             launch_pdl(k_conv_tc<1, CHUNK, MD>, g, kTcThreads, smem, st, ctx, level, a);
             break;
         case 2:
-            set_smem_attr<2, CHUNK, MD>();
             launch_pdl(k_conv_tc<2, CHUNK, MD>, g, kTcThreads, smem, st, ctx, level, a);
             break;
         case 3:
-            set_smem_attr<3, CHUNK, MD>();
             launch_pdl(k_conv_tc<3, CHUNK, MD>, g, kTcThreads, smem, st, ctx, level, a);
             break;
         default:
-            set_smem_attr<4, CHUNK, MD>();
             launch_pdl(k_conv_tc<4, CHUNK, MD>, g, kTcThreads, smem, st, ctx, level, a);
             break;
     }
@@ -559,6 +546,20 @@ bool conv_tc_eligible(const DevCtx& ctx, uint64_t smallest) {
     return up <= kTcMaxTargets && ctx.L <= kTcMaxTargets &&
            tc_smem_bytes((ctx.alpha + 3) / 4, up, false) <= kTcSmemCap &&
            tc_smem_bytes((ctx.K + 3) / 4, ctx.L, true) <= kTcSmemCap;
+}
+
+// shared-memory opt-in of every instance, on the current device
+cudaError_t conv_tc_prepare() {
+    cudaError_t e = cudaSuccess;
+    auto opt_in = [&](auto... k) {
+        for (cudaError_t r : {cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemCap)...})
+            if (e == cudaSuccess) e = r;
+    };
+    opt_in(k_conv_tc<1, 16, false>, k_conv_tc<2, 16, false>, k_conv_tc<3, 16, false>, k_conv_tc<4, 16, false>);
+    opt_in(k_conv_tc<1, 32, false>, k_conv_tc<2, 32, false>, k_conv_tc<3, 32, false>, k_conv_tc<4, 32, false>);
+    opt_in(k_conv_tc<1, 16, true>, k_conv_tc<2, 16, true>, k_conv_tc<3, 16, true>, k_conv_tc<4, 16, true>);
+    opt_in(k_conv_tc<1, 32, true>, k_conv_tc<2, 32, true>, k_conv_tc<3, 32, true>, k_conv_tc<4, 32, true>);
+    return e;
 }
 
 bool conv_tc_supported(const DevCtx& ctx) { return ctx.tc_btab != nullptr; }
