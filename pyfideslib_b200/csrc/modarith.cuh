@@ -3,7 +3,7 @@
 //
 // All products here are on the integer pipes (IMAD); nothing is approximated.
 // (The NTT also has exact double-precision butterflies for primes below
-// 2^50, in ntt.cu.)
+// 2^50, in ntt_kernels.cuh.)
 // Canonical residues live in [0, p); the transforms keep Harvey's lazy
 // ranges [0, 2p) / [0, 4p) internally and reduce at the end.
 //
@@ -46,7 +46,7 @@ struct PrimeConst {
 };
 
 // Forward transforms of primes below this bound run their butterflies on the
-// FP64 pipes (residues held exactly as doubles, see ntt.cu).
+// FP64 pipes (residues held exactly as doubles, see ntt_kernels.cuh).
 constexpr uint64_t kFpPrimeBound = 1ull << 50;
 
 // floor(w * 2^64 / p), host only (needs a 128-bit division).
