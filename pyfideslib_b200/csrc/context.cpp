@@ -540,7 +540,7 @@ fides_status build_context(fides_ctx* c, const fides_params* prm) {
             if (cudaMemcpy(tb + bytes, offs.data(), obytes, cudaMemcpyHostToDevice) == cudaSuccess) {
                 d.tc_btab = tb;
                 d.tc_boff = (const uint64_t*)(tb + bytes);
-                if (conv_tc_prepare() != cudaSuccess)
+                if (conv_tc_prepare(d) != cudaSuccess)
                     return set_err(c, FIDES_CUDA_ERR, "shared-memory opt-in of the conversions failed");
                 conv_tc_build_tables(d, c->st);
                 if (cudaStreamSynchronize(c->st) != cudaSuccess) return set_err(c, FIDES_CUDA_ERR, "table build failed");

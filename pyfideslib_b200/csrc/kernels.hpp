@@ -150,7 +150,7 @@ constexpr int kConvVariants = 5;  // see DevCtx::conv_variant
 // (conv_tc.cu); chunk = targets per MMA (32 or 16)
 bool conv_tc_eligible(const DevCtx& ctx, uint64_t smallest);  // shapes and moduli the kernels handle
 bool conv_tc_supported(const DevCtx& ctx);                     // eligible and the B tables built
-cudaError_t conv_tc_prepare();                                 // per device, before their first launch
+cudaError_t conv_tc_prepare(const DevCtx& ctx);                // per context, before its first launch
 // byte offsets of the per-(level, digit) and per-(level, fused) B matrices
 size_t conv_tc_table_layout(const DevCtx& ctx, std::vector<uint64_t>& offs);
 void conv_tc_build_tables(const DevCtx& ctx, cudaStream_t st);
